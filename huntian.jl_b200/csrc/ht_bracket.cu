@@ -19,11 +19,10 @@
 //   mlp_infer_tc_kernel  inference, 128 peaks per CTA tile: every layer a tcgen05.mma chain
 //                        from shared memory into tensor memory, read back per row
 //                        (tcgen05.ld), bias + ReLU + BF16 as the next layer's operand
-//   gemm_bf16_kernel     generic C = op(A) op(B) (BF16 in, FP32 out, mma.sync m16n8k16)
-//                        for training (offline, not on the step):
-//                        forward products, activation gradients and weight gradients
-//   small elementwise kernels for bias/ReLU, the pinball-loss gradient, ReLU backward,
-//   bias gradients and Adam.
+//   train_grad_kernel    training (offline, not on the step): forward, pinball loss,
+//                        backward and the weight gradients of 128-sample tiles, one CTA
+//                        partial each; train_reduce_kernel adds the partials
+//   adam_kernel          the optimiser step
 #include <cuda_bf16.h>
 #include <math.h>
 
@@ -413,140 +412,328 @@ __global__ void __launch_bounds__(kTcRows) mlp_infer_tc_kernel(const MlpW w,
 
 // --------------------------------------------------------------- training ----
 //
-// C[M x N] (FP32, row stride N) = op(A) op(B): A element (m, k) at A[m sam + k sak], B
-// element (k, n) at B[k sbk + n sbn], both BF16.  A CTA computes a 64 x 64 tile with four
-// warps of 32 x 32 (2 x 4 mma tiles); K advances in slices of 16 staged in shared memory
-// (zero-filled outside the matrices).  The same kernel serves the forward products
-// (X W^T), the activation gradients (dZ W) and the weight gradients (dZ^T H, K = batch).
+// Gradient of the mean pinball loss in one kernel.  A CTA of 8 warps takes tiles of 128
+// samples, persistent over the tiles; a warp carries 16 samples through the whole network
+// in registers (mma.sync m16n8k16: the accumulator of one layer is, rounded to BF16, the A
+// operand of the next), forward and back, and leaves the BF16 activations and dZ of its
+// rows in shared memory.  The CTA then adds dZ^T H of the tile to the weight gradients,
+// which stay in the warps' accumulators over all tiles (16 x 32 of dW2 and dW3, 16 x 8 of
+// dW1 and dW4 each; ldmatrix.trans gives both operands with the samples as K).  Every CTA
+// writes one partial gradient and train_reduce_kernel adds them in CTA order, so the
+// result does not depend on timing.  What bounds it is the chain of dependent layers of a
+// tile, not bytes (68 B a sample) or MMAs.
+//
+// The samples are the K of the weight gradients: a GEMM tiled over the 64 x 64 output ran
+// them on one CTA, 26.1 ms of the 26.3 ms of a 65,536-sample gradient and Adam step; that
+// step takes 44 us with this kernel (four tiles per CTA, one CTA per SM: 175 KB of shared
+// memory and 255 registers hold a tile's matrices and every accumulator).
 
-constexpr int kTM = 64, kTN = 64, kTK = 16, kPadK = 24;
+constexpr int kTrRows = 128, kTrWarps = 8, kTrThreads = 32 * kTrWarps;
+constexpr int kTrS = 72, kTrSn = 24;      // row strides (BF16) of 64- and 16-wide matrices:
+                                          // 36 and 12 words, conflict-free fragment reads
+constexpr int kTrPart = HT_BRACKET_NPARAMS + 8;   // a CTA's partial: gradient, then the loss
 
-__global__ void __launch_bounds__(128) gemm_bf16_kernel(
-    const __nv_bfloat16* __restrict__ A, long long sam, long long sak,
-    const __nv_bfloat16* __restrict__ B, long long sbk, long long sbn, float* __restrict__ C,
-    int M, int N, int K) {
-    __shared__ __align__(16) __nv_bfloat16 As[kTM][kPadK];
-    __shared__ __align__(16) __nv_bfloat16 Bs[kTN][kPadK];
+// Shared-memory layout (bytes from the dynamic base).
+constexpr int kTrBig = kTrRows * kTrS * 2, kTrNarrow = kTrRows * kTrSn * 2;
+constexpr int kTrOffX = 0, kTrOffY = kTrOffX + kTrNarrow, kTrOffH = kTrOffY + kTrNarrow,
+              kTrOffD = kTrOffH + 3 * kTrBig, kTrOffW1 = kTrOffD + 3 * kTrBig,
+              kTrOffW = kTrOffW1 + kHid * kTrSn * 2,          // W2, W3 [out][in]
+              kTrOffWT = kTrOffW + 2 * kHid * kTrS * 2,       // W2, W3 [in][out]
+              kTrOffW4 = kTrOffWT + 2 * kHid * kTrS * 2,      // W4 [8][in]
+              kTrOffW4T = kTrOffW4 + 8 * kTrS * 2,            // W4 [in][16]
+              kTrOffB = kTrOffW4T + kHid * kTrSn * 2,         // b1 b2 b3 [64] b4 [8] FP32
+              kTrOffR = kTrOffB + 200 * 4,                    // [8 warps][200] bias sums
+              kTrSmem = kTrOffR + kTrWarps * 200 * 4;
+static_assert(kTrSmem <= 227 * 1024, "one CTA per SM");
+
+__device__ __forceinline__ void ldmatrix4_trans(unsigned (&r)[4], const void* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(htasync::smem_addr(p)) : "memory");
+}
+
+__device__ __forceinline__ unsigned ld32(const __nv_bfloat16* p) {
+    return *reinterpret_cast<const unsigned*>(p);
+}
+
+// c[j] (8 columns 8 j .. 8 j + 7, j < NJ) += A B over KS steps of 16, B (k, n) at
+// W[n * stride + k].
+template <int KS, int NJ>
+__device__ __forceinline__ void warp_gemm(float (&c)[NJ][4], const unsigned (&a)[KS][4],
+                                          const __nv_bfloat16* W, int stride, int g, int t) {
+#pragma unroll
+    for (int s = 0; s < KS; ++s)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+            const __nv_bfloat16* p = W + (8 * j + g) * stride + 16 * s + 2 * t;
+            mma_bf16(c[j], a[s], ld32(p), ld32(p + 8));
+        }
+}
+
+// The warp's 16 x 64 values c, rounded to BF16, as the next product's A operand and in
+// rows g and g + 8 of S.
+__device__ __forceinline__ void to_operand(const float (&c)[8][4], unsigned (&a)[4][4],
+                                           __nv_bfloat16* S, int g, int t) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const unsigned lo = pack_bf16(c[j][0], c[j][1]), hi = pack_bf16(c[j][2], c[j][3]);
+        a[j >> 1][2 * (j & 1)] = lo;
+        a[j >> 1][2 * (j & 1) + 1] = hi;
+        *reinterpret_cast<unsigned*>(S + g * kTrS + 8 * j + 2 * t) = lo;
+        *reinterpret_cast<unsigned*>(S + (g + 8) * kTrS + 8 * j + 2 * t) = hi;
+    }
+}
+
+// z = c + b, kept positions of z > 0, relu; then as to_operand.
+__device__ __forceinline__ unsigned activate(float (&c)[8][4], const float* b,
+                                             unsigned (&a)[4][4], __nv_bfloat16* S, int g,
+                                             int t) {
+    unsigned pos = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float z = c[j][e] + b[8 * j + 2 * t + (e & 1)];
+            if (z > 0.f) pos |= 1u << (4 * j + e);
+            c[j][e] = fmaxf(z, 0.f);
+        }
+    to_operand(c, a, S, g, t);
+    return pos;
+}
+
+// dZ = dH where z > 0, added to the column sums; then as to_operand.
+__device__ __forceinline__ void relu_back(float (&c)[8][4], unsigned pos, float (&db)[16],
+                                          unsigned (&a)[4][4], __nv_bfloat16* S, int g,
+                                          int t) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (!((pos >> (4 * j + e)) & 1u)) c[j][e] = 0.f;
+        db[2 * j] += c[j][0] + c[j][2];
+        db[2 * j + 1] += c[j][1] + c[j][3];
+    }
+    to_operand(c, a, S, g, t);
+}
+
+template <int NJ>
+__device__ __forceinline__ void clear(float (&c)[NJ][4]) {
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) c[j][e] = 0.f;
+}
+
+__global__ void __launch_bounds__(kTrThreads, 1) train_grad_kernel(
+    const MlpW w, const float* __restrict__ F, const float* __restrict__ tgt, long long n,
+    float* __restrict__ part) {
+    extern __shared__ __align__(128) unsigned char tsm[];
+    auto mat = [&](int off) { return reinterpret_cast<__nv_bfloat16*>(tsm + off); };
+    __nv_bfloat16 *Xs = mat(kTrOffX), *Ys = mat(kTrOffY), *W1 = mat(kTrOffW1),
+                  *W4 = mat(kTrOffW4), *W4T = mat(kTrOffW4T);
+    auto Hs = [&](int l) { return mat(kTrOffH + l * kTrBig); };
+    auto Ds = [&](int l) { return mat(kTrOffD + l * kTrBig); };
+    auto Wm = [&](int l) { return mat(kTrOffW + (l - 1) * kHid * kTrS * 2); };   // l = 1, 2
+    auto WT = [&](int l) { return mat(kTrOffWT + (l - 1) * kHid * kTrS * 2); };
+    float* bias = reinterpret_cast<float*>(tsm + kTrOffB);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const int m0 = blockIdx.y * kTM, n0 = blockIdx.x * kTN;
-    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
-    float acc[2][4][4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
     const __nv_bfloat16 zero = __float2bfloat16(0.f);
-    for (int k0 = 0; k0 < K; k0 += kTK) {
-        for (int e = tid; e < kTM * kTK; e += blockDim.x) {
-            const int r = e / kTK, c = e % kTK;
-            const int m = m0 + r, k = k0 + c;
-            As[r][c] = (m < M && k < K) ? A[(long long)m * sam + (long long)k * sak] : zero;
-            const int n = n0 + r;
-            Bs[r][c] = (n < N && k < K) ? B[(long long)k * sbk + (long long)n * sbn] : zero;
+    for (int e = tid; e < kHid * kHid; e += kTrThreads) {
+        const int o = e / kHid, i = e % kHid;
+        const __nv_bfloat16 v2 = w.W2[e], v3 = w.W3[e];
+        Wm(1)[o * kTrS + i] = v2;
+        WT(1)[i * kTrS + o] = v2;
+        Wm(2)[o * kTrS + i] = v3;
+        WT(2)[i * kTrS + o] = v3;
+    }
+    for (int e = tid; e < kHid * kIn; e += kTrThreads) {
+        const int o = e / kIn, i = e % kIn;
+        W1[o * kTrSn + i] = w.W1[e];
+        W4T[o * kTrSn + i] = i < 2 ? w.W4[i * kHid + o] : zero;   // (in, out): two outputs
+    }
+    for (int e = tid; e < 8 * kHid; e += kTrThreads)
+        W4[(e / kHid) * kTrS + e % kHid] = e < 2 * kHid ? w.W4[e] : zero;
+    for (int e = tid; e < kTrRows * kTrSn; e += kTrThreads) Ys[e] = zero;
+    if (tid < kHid) {
+        bias[tid] = w.b1[tid];
+        bias[kHid + tid] = w.b2[tid];
+        bias[2 * kHid + tid] = w.b3[tid];
+    }
+    if (tid < 2) bias[3 * kHid + tid] = w.b4[tid];
+    __syncthreads();
+
+    // weight-gradient accumulators of this warp: rows (outputs) 16 mi .. 16 mi + 15
+    const int mi = warp >> 1, nh = warp & 1;
+    float g2[4][4], g3[4][4], g1[1][4], g4[1][4];   // columns 32 nh.., 32 nh.., 8 nh.., 8 warp..
+    clear(g2);
+    clear(g3);
+    clear(g1);
+    clear(g4);
+    float db[3][16], db4[2] = {0.f, 0.f}, loss = 0.f;
+#pragma unroll
+    for (int l = 0; l < 3; ++l)
+#pragma unroll
+        for (int i = 0; i < 16; ++i) db[l][i] = 0.f;
+    const float inv = 1.0f / (float)n;
+    const int r0 = 16 * warp;                       // the warp's rows of the tile
+    const long long ntiles = (n + kTrRows - 1) / kTrRows;
+    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const long long ra = tile * kTrRows + r0 + g, rb = ra + 8;   // this thread's samples
+        unsigned a[4][4], x[1][4];
+        float c[8][4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {               // x[0][q]: row ra / rb, inputs k, k + 1
+            const long long r = (q & 1) ? rb : ra;
+            const int k = 2 * t + 8 * (q >> 1);
+            float v0 = 0.f, v1 = 0.f;
+            if (r < n) {
+                v0 = (__ldg(F + r * kIn + k) - __ldg(w.mean + k)) * __ldg(w.istd + k);
+                v1 = (__ldg(F + r * kIn + k + 1) - __ldg(w.mean + k + 1)) * __ldg(w.istd + k + 1);
+            }
+            x[0][q] = pack_bf16(v0, v1);
+            *reinterpret_cast<unsigned*>(Xs + (r0 + g + 8 * (q & 1)) * kTrSn + k) = x[0][q];
         }
-        __syncthreads();
+        // forward
+        unsigned pos[3];
+        clear(c);
+        warp_gemm<1, 8>(c, x, W1, kTrSn, g, t);
+        pos[0] = activate(c, bias, a, Hs(0) + r0 * kTrS, g, t);
+        clear(c);
+        warp_gemm<4, 8>(c, a, Wm(1), kTrS, g, t);
+        pos[1] = activate(c, bias + kHid, a, Hs(1) + r0 * kTrS, g, t);
+        clear(c);
+        warp_gemm<4, 8>(c, a, Wm(2), kTrS, g, t);
+        pos[2] = activate(c, bias + 2 * kHid, a, Hs(2) + r0 * kTrS, g, t);
+        float y[1][4];
+        clear(y);
+        warp_gemm<4, 1>(y, a, W4, kTrS, g, t);
+        // pinball loss of the two quantiles (tau 0.1 and 0.9): columns 0, 1 sit in lanes t = 0
+        unsigned dy[1][4] = {{0u, 0u, 0u, 0u}};
+        if (t == 0) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            unsigned a[4];
-            const int r = wm + 16 * i + g;
-            a[0] = *reinterpret_cast<const unsigned*>(&As[r][2 * t]);
-            a[1] = *reinterpret_cast<const unsigned*>(&As[r + 8][2 * t]);
-            a[2] = *reinterpret_cast<const unsigned*>(&As[r][2 * t + 8]);
-            a[3] = *reinterpret_cast<const unsigned*>(&As[r + 8][2 * t + 8]);
+            for (int h = 0; h < 2; ++h) {
+                const long long r = h ? rb : ra;
+                float gq[2] = {0.f, 0.f};
+                if (r < n) {
+                    const float target = __ldg(tgt + r);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int nn = wn + 8 * j + g;
-                const unsigned b0 = *reinterpret_cast<const unsigned*>(&Bs[nn][2 * t]);
-                const unsigned b1 = *reinterpret_cast<const unsigned*>(&Bs[nn][2 * t + 8]);
-                mma_bf16(acc[i][j], a, b0, b1);
+                    for (int q = 0; q < 2; ++q) {
+                        const float tau = q ? 0.9f : 0.1f;
+                        const float d = target - (y[0][2 * h + q] + bias[3 * kHid + q]);
+                        loss += d > 0.f ? tau * d : (tau - 1.f) * d;
+                        gq[q] = (d > 0.f ? -tau : 1.f - tau) * inv;
+                        db4[q] += gq[q];
+                    }
+                }
+                dy[0][h] = pack_bf16(gq[0], gq[1]);
+                *reinterpret_cast<unsigned*>(Ys + (r0 + g + 8 * h) * kTrSn) = dy[0][h];
             }
         }
+        __syncwarp();
+        // backward
+        clear(c);
+        warp_gemm<1, 8>(c, dy, W4T, kTrSn, g, t);
+        relu_back(c, pos[2], db[2], a, Ds(2) + r0 * kTrS, g, t);
+        clear(c);
+        warp_gemm<4, 8>(c, a, WT(2), kTrS, g, t);
+        relu_back(c, pos[1], db[1], a, Ds(1) + r0 * kTrS, g, t);
+        clear(c);
+        warp_gemm<4, 8>(c, a, WT(1), kTrS, g, t);
+        relu_back(c, pos[0], db[0], a, Ds(0) + r0 * kTrS, g, t);
         __syncthreads();
-    }
+        // weight gradients: K = the tile's 128 samples
+        const int lr = lane & 7, q = lane >> 3;
+        const int ka = lr + 8 * (q >> 1), ma = 8 * (q & 1);   // A: (k, m) blocks 00 01 10 11
+        const int kb = lr + 8 * (q & 1), nb = 8 * (q >> 1);   // B: (k, n) blocks 00 10 01 11
+#pragma unroll 2
+        for (int k0 = 0; k0 < kTrRows; k0 += 16) {
+            unsigned A[4], B[4];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+            for (int l = 1; l < 3; ++l) {
+                ldmatrix4_trans(A, Ds(l) + (k0 + ka) * kTrS + 16 * mi + ma);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int r = m0 + wm + 16 * i + g, c = n0 + wn + 8 * j + 2 * t;
-            if (r < M && c < N) C[(long long)r * N + c] = acc[i][j][0];
-            if (r < M && c + 1 < N) C[(long long)r * N + c + 1] = acc[i][j][1];
-            if (r + 8 < M && c < N) C[(long long)(r + 8) * N + c] = acc[i][j][2];
-            if (r + 8 < M && c + 1 < N) C[(long long)(r + 8) * N + c + 1] = acc[i][j][3];
+                for (int h = 0; h < 2; ++h) {
+                    ldmatrix4_trans(B, Hs(l - 1) + (k0 + kb) * kTrS + 32 * nh + 16 * h + nb);
+                    auto& acc = l == 1 ? g2 : g3;
+                    mma_bf16(acc[2 * h], A, B[0], B[1]);
+                    mma_bf16(acc[2 * h + 1], A, B[2], B[3]);
+                }
+            }
+            ldmatrix4_trans(A, Ds(0) + (k0 + ka) * kTrS + 16 * mi + ma);
+            ldmatrix4_trans(B, Xs + (k0 + kb) * kTrSn + nb);
+            mma_bf16(g1[0], A, nh ? B[2] : B[0], nh ? B[3] : B[1]);
+            ldmatrix4_trans(A, Ys + (k0 + ka) * kTrSn + ma);
+            ldmatrix4_trans(B, Hs(2) + (k0 + kb) * kTrS + 16 * (warp >> 1) + nb);
+            mma_bf16(g4[0], A, nh ? B[2] : B[0], nh ? B[3] : B[1]);
         }
-}
-
-// X = bf16((F - mean) * istd), [M x 16]
-__global__ void standardise_kernel(const float* __restrict__ F, const float* __restrict__ mean,
-                                   const float* __restrict__ istd, long long M,
-                                   __nv_bfloat16* __restrict__ X) {
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= M * kIn) return;
-    const int c = (int)(e % kIn);
-    X[e] = __float2bfloat16((F[e] - mean[c]) * istd[c]);
-}
-
-// Z += b (in place); H = bf16(relu(Z)) when H is given
-__global__ void bias_act_kernel(float* __restrict__ Z, const float* __restrict__ b, long long M,
-                                int N, __nv_bfloat16* __restrict__ H) {
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= M * N) return;
-    const float z = Z[e] + b[e % N];
-    Z[e] = z;
-    if (H) H[e] = __float2bfloat16(fmaxf(z, 0.f));
-}
-
-// Pinball loss of the two quantile outputs (tau 0.1 and 0.9) against the target; dY / M
-// as BF16 [M x 16] (columns 2..15 zero) and FP32 [M x 2]; loss summed into *loss.
-__global__ void pinball_kernel(const float* __restrict__ Y, const float* __restrict__ tgt,
-                               long long M, __nv_bfloat16* __restrict__ dYb,
-                               float* __restrict__ dYf, float* __restrict__ loss) {
-    const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    float l = 0.f;
-    if (r < M) {
-        const float tau[2] = {0.1f, 0.9f};
-        const float inv = 1.0f / (float)M;
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const float d = tgt[r] - Y[r * 2 + q];
-            l += d > 0.f ? tau[q] * d : (tau[q] - 1.f) * d;
-            const float gq = (d > 0.f ? -tau[q] : 1.f - tau[q]) * inv;
-            dYf[r * 2 + q] = gq;
-            dYb[r * kIn + q] = __float2bfloat16(gq);
-        }
-#pragma unroll
-        for (int c = 2; c < kIn; ++c) dYb[r * kIn + c] = __float2bfloat16(0.f);
+        __syncthreads();   // the tile's matrices have been read
     }
-    for (int o = 16; o >= 1; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, l / (float)M);
-}
 
-// dZ = dH * (Z > 0): FP32 in place and a BF16 copy
-__global__ void relu_back_kernel(float* __restrict__ dH, const float* __restrict__ Z, long long M,
-                                 int N, __nv_bfloat16* __restrict__ dZb) {
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= M * N) return;
-    const float d = Z[e] > 0.f ? dH[e] : 0.f;
-    dH[e] = d;
-    dZb[e] = __float2bfloat16(d);
-}
-
-// db[n] = sum_m dZ[m][n] (one block per column, fixed reduction order)
-__global__ void colsum_kernel(const float* __restrict__ dZ, long long M, int N,
-                              float* __restrict__ db) {
-    __shared__ float red[256];
-    const int n = blockIdx.x;
-    float s = 0.f;
-    for (long long m = threadIdx.x; m < M; m += blockDim.x) s += dZ[m * N + n];
-    red[threadIdx.x] = s;
+    // this CTA's partial gradient: W1 [64x16] W2 W3 [64x64] W4 [8x64] b1 b2 b3 [64] b4 [8]
+    float* P = part + (size_t)blockIdx.x * kTrPart;
+    auto put = [&](float* M, int ld, int m0, int n0, const float (&v)[4], int rows) {
+        if (m0 + g < rows)
+            *reinterpret_cast<float2*>(M + (m0 + g) * ld + n0 + 2 * t) = make_float2(v[0], v[1]);
+        if (m0 + g + 8 < rows)
+            *reinterpret_cast<float2*>(M + (m0 + g + 8) * ld + n0 + 2 * t) =
+                make_float2(v[2], v[3]);
+    };
+    put(P, kIn, 16 * mi, 8 * nh, g1[0], kHid);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        put(P + 1024, kHid, 16 * mi, 32 * nh + 8 * j, g2[j], kHid);
+        put(P + 5120, kHid, 16 * mi, 32 * nh + 8 * j, g3[j], kHid);
+    }
+    if (g >= 2) g4[0][0] = g4[0][1] = 0.f;   // W4's padding rows, whatever the activations
+    put(P + 9216, kHid, 0, 8 * warp, g4[0], 8);
+    // bias gradients and the loss: over the rows of the warp, then over the warps in order
+    float* R = reinterpret_cast<float*>(tsm + kTrOffR) + warp * 200;
+#pragma unroll
+    for (int l = 0; l < 3; ++l)
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            float v = db[l][i];
+            for (int o = 4; o <= 16; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (g == 0) R[l * kHid + 8 * (i >> 1) + 2 * t + (i & 1)] = v;
+        }
+    float v[3] = {db4[0], db4[1], loss};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        for (int o = 4; o <= 16; o <<= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+        if (lane == 0) R[192 + i] = v[i];
+    }
     __syncthreads();
-    for (int o = blockDim.x / 2; o >= 1; o >>= 1) {
-        if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-        __syncthreads();
+    const float* R0 = reinterpret_cast<const float*>(tsm + kTrOffR);
+    if (tid < 195) {
+        float s = 0.f;
+        for (int k = 0; k < kTrWarps; ++k) s += R0[k * 200 + tid];
+        P[tid < 194 ? 9728 + tid : HT_BRACKET_NPARAMS] = s;
+    } else if (tid < 201) {
+        P[9728 + tid - 1] = 0.f;   // b4's padding
     }
-    if (threadIdx.x == 0) db[n] = red[0];
+}
+
+// grads[i] = the sum of the CTAs' partials in order (8 strided sums, then those in order);
+// loss = its sum / n.  A block takes 32 neighbouring values.
+__global__ void __launch_bounds__(256) train_reduce_kernel(const float* __restrict__ part,
+                                                           int ctas, long long n,
+                                                           float* __restrict__ grads,
+                                                           float* __restrict__ loss) {
+    __shared__ float red[8][33];
+    const int c = threadIdx.x & 31, k = threadIdx.x >> 5, i = blockIdx.x * 32 + c;
+    float s = 0.f;
+    if (i <= HT_BRACKET_NPARAMS)
+        for (int b = k; b < ctas; b += 8) s += __ldg(part + (size_t)b * kTrPart + i);
+    red[k][c] = s;
+    __syncthreads();
+    if (k == 0 && i <= HT_BRACKET_NPARAMS) {
+        s = 0.f;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) s += red[q][c];
+        if (i < HT_BRACKET_NPARAMS) grads[i] = s;
+        else *loss = s / (float)n;
+    }
 }
 
 // Adam on the packed FP32 parameters; writes the BF16 weights and FP32 biases of `out`.
@@ -598,17 +785,6 @@ MlpW mlp_of(const ht_bracket_model* m) {
     w.b1 = m->b1; w.b2 = m->b2; w.b3 = m->b3; w.b4 = m->b4;
     w.mean = m->mean; w.istd = m->istd;
     return w;
-}
-
-int launch_gemm(const __nv_bfloat16* A, long long sam, long long sak, const __nv_bfloat16* B,
-                long long sbk, long long sbn, float* C, long long M, int N, long long K,
-                cudaStream_t st) {
-    if (M > 0x7fffffffLL || K > 0x7fffffffLL)
-        return ht_fail(HT_ERR_CAPACITY, "bracket GEMM: dimension too large");
-    dim3 grid((unsigned)((N + kTN - 1) / kTN), (unsigned)((M + kTM - 1) / kTM));
-    gemm_bf16_kernel<<<grid, 128, 0, st>>>(A, sam, sak, B, sbk, sbn, C, (int)M, N, (int)K);
-    HT_CUDA_TRY(cudaGetLastError(), "gemm_bf16_kernel launch");
-    return HT_OK;
 }
 
 unsigned blocks_for(long long n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -675,68 +851,19 @@ extern "C" HT_API int ht_bracket_grad(ht_ctx* ctx, const ht_bracket_model* m,
     if (n < 1 || n > (1LL << 24)) return ht_fail(HT_ERR_INVALID, "ht_bracket_grad: need 1 <= n <= 2^24");
     HT_CUDA_TRY(cudaSetDevice(ctx->device), "cudaSetDevice");
     cudaStream_t st = (cudaStream_t)stream;
-    // workspace per row: X (16 bf16), Z1..Z3 (64 f32), H1..H3 (64 bf16), Y (2 f32),
-    // dYb (16 bf16), dYf (2 f32), dH (64 f32), dZb (64 bf16)
-    const size_t row = 16 * 2 + 3 * 64 * 4 + 3 * 64 * 2 + 8 + 16 * 2 + 8 + 64 * 4 + 64 * 2;
-    rc = ht_grow(&ctx->d_mlp_ws, &ctx->mlp_ws_bytes, row * (size_t)n + 4096, "bracket training workspace");
+    const long long tiles = (n + kTrRows - 1) / kTrRows;
+    const int ctas = (int)std::min<long long>(tiles, ctx->num_sms);
+    rc = ht_grow(&ctx->d_mlp_ws, &ctx->mlp_ws_bytes, (size_t)ctas * kTrPart * sizeof(float),
+                 "bracket training workspace");
     if (rc != HT_OK) return rc;
-    char* w = (char*)ctx->d_mlp_ws;
-    auto take = [&](size_t bytes) { char* p = w; w += (bytes + 255) / 256 * 256; return p; };
-    __nv_bfloat16* X = (__nv_bfloat16*)take((size_t)n * 16 * 2);
-    float* Z[3]; __nv_bfloat16* H[3];
-    for (int l = 0; l < 3; ++l) { Z[l] = (float*)take((size_t)n * 64 * 4); H[l] = (__nv_bfloat16*)take((size_t)n * 64 * 2); }
-    float* Y = (float*)take((size_t)n * 2 * 4);
-    __nv_bfloat16* dYb = (__nv_bfloat16*)take((size_t)n * 16 * 2);
-    float* dYf = (float*)take((size_t)n * 2 * 4);
-    float* dH = (float*)take((size_t)n * 64 * 4);
-    __nv_bfloat16* dZb = (__nv_bfloat16*)take((size_t)n * 64 * 2);
-    const __nv_bfloat16* W[4] = {(const __nv_bfloat16*)m->W1, (const __nv_bfloat16*)m->W2,
-                                 (const __nv_bfloat16*)m->W3, (const __nv_bfloat16*)m->W4};
-    const float* bias[4] = {m->b1, m->b2, m->b3, m->b4};
-    // gradient layout (FP32): dW1 [64x16] dW2 dW3 [64x64] dW4 [8x64] db1 db2 db3 [64] db4 [8]
-    float* gW[4] = {d_grads, d_grads + 1024, d_grads + 5120, d_grads + 9216};
-    float* gb[4] = {d_grads + 9728, d_grads + 9792, d_grads + 9856, d_grads + 9920};
-    HT_CUDA_TRY(cudaMemsetAsync(d_grads, 0, 9928 * sizeof(float), st), "grad reset");
-    HT_CUDA_TRY(cudaMemsetAsync(d_loss, 0, sizeof(float), st), "loss reset");
-    const int T = 256;
-    standardise_kernel<<<blocks_for(n * kIn, T), T, 0, st>>>(d_feat, m->mean, m->istd, n, X);
-    HT_CUDA_TRY(cudaGetLastError(), "standardise_kernel launch");
-    // forward: Z_l = H_{l-1} W_l^T + b_l, H_l = relu(Z_l)
-    const __nv_bfloat16* in = X;
-    int K = kIn;
-    for (int l = 0; l < 3; ++l) {
-        if ((rc = launch_gemm(in, K, 1, W[l], 1, K, Z[l], n, kHid, K, st)) != HT_OK) return rc;
-        bias_act_kernel<<<blocks_for(n * kHid, T), T, 0, st>>>(Z[l], bias[l], n, kHid, H[l]);
-        HT_CUDA_TRY(cudaGetLastError(), "bias_act_kernel launch");
-        in = H[l];
-        K = kHid;
-    }
-    if ((rc = launch_gemm(H[2], kHid, 1, W[3], 1, kHid, Y, n, 2, kHid, st)) != HT_OK) return rc;
-    bias_act_kernel<<<blocks_for(n * 2, T), T, 0, st>>>(Y, bias[3], n, 2, nullptr);
-    HT_CUDA_TRY(cudaGetLastError(), "bias_act_kernel launch");
-    pinball_kernel<<<blocks_for(n, T), T, 0, st>>>(Y, d_target, n, dYb, dYf, d_loss);
-    HT_CUDA_TRY(cudaGetLastError(), "pinball_kernel launch");
-    // output layer: dW4 = dY^T H3 (rows 0..1), db4, dH3 = dY W4
-    if ((rc = launch_gemm(dYb, 1, kIn, H[2], kHid, 1, gW[3], 2, kHid, n, st)) != HT_OK) return rc;
-    colsum_kernel<<<2, 256, 0, st>>>(dYf, n, 2, gb[3]);
-    HT_CUDA_TRY(cudaGetLastError(), "colsum_kernel launch");
-    if ((rc = launch_gemm(dYb, kIn, 1, W[3], kHid, 1, dH, n, kHid, 2, st)) != HT_OK) return rc;
-    for (int l = 2; l >= 0; --l) {
-        relu_back_kernel<<<blocks_for(n * kHid, T), T, 0, st>>>(dH, Z[l], n, kHid, dZb);
-        HT_CUDA_TRY(cudaGetLastError(), "relu_back_kernel launch");
-        colsum_kernel<<<kHid, 256, 0, st>>>(dH, n, kHid, gb[l]);
-        HT_CUDA_TRY(cudaGetLastError(), "colsum_kernel launch");
-        const __nv_bfloat16* prev = l > 0 ? H[l - 1] : X;
-        const int Kp = l > 0 ? kHid : kIn;
-        // dW_l = dZ_l^T prev : (64 x Kp), K = n
-        if ((rc = launch_gemm(dZb, 1, kHid, prev, Kp, 1, gW[l], kHid, Kp, n, st)) != HT_OK) return rc;
-        if (l > 0) {
-            // dH_{l-1} = dZ_l W_l : (n x 64), K = 64
-            if ((rc = launch_gemm(dZb, kHid, 1, W[l], kHid, 1, dH, n, kHid, kHid, st)) != HT_OK)
-                return rc;
-        }
-    }
-    ctx->last_kernels = 0;
+    float* part = (float*)ctx->d_mlp_ws;
+    HT_CUDA_TRY(cudaFuncSetAttribute(train_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrSmem), "train_grad smem");
+    train_grad_kernel<<<ctas, kTrThreads, kTrSmem, st>>>(mlp_of(m), d_feat, d_target, n, part);
+    HT_CUDA_TRY(cudaGetLastError(), "train_grad_kernel launch");
+    train_reduce_kernel<<<blocks_for(HT_BRACKET_NPARAMS + 1, 32), 256, 0, st>>>(part, ctas, n,
+                                                                               d_grads, d_loss);
+    HT_CUDA_TRY(cudaGetLastError(), "train_reduce_kernel launch");
+    ctx->last_kernels = 2;
     return HT_OK;
 }
 

@@ -87,6 +87,32 @@ def test_gradient_check_against_cpu(ht, finder):
     assert np.all(g[o + 128:o + 512] == 0)
 
 
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 148 * 128 + 1])
+def test_gradient_at_tile_edges(ht, finder, n):
+    """Whole and partial 128-sample tiles, and more tiles than CTAs.  The relative error of a
+    block is that of BF16 operands whose rounding a different FP32 order can move (half an
+    ulp, 2^-9, per factor of the products)."""
+    br = ht.bracket
+    rng = np.random.default_rng(100 + n)
+    p, mean, istd = _random_model(ht, 4)
+    F = _features(rng, n)
+    ref_y, _ = br.reference_forward(p, mean, istd, F)
+    t = (ref_y.numpy().mean(1) + rng.normal(0, 1.0, n)).astype(np.float32)
+    model = br.BracketModel(p, mean, istd)
+    args = (torch.as_tensor(F, device="cuda"), torch.as_tensor(t, device="cuda"))
+    g, loss = br.grad(finder, model, *args)
+    again, _ = br.grad(finder, model, *args)
+    assert torch.equal(g, again)
+    ref = br.reference_grad(p, mean, istd, F, t)
+    for name, (o, s) in br.OFFSETS.items():
+        k = int(np.prod(s))
+        a, b = g[o:o + k].cpu().numpy(), ref[o:o + k]
+        assert np.linalg.norm(a - b) <= 2e-2 * np.linalg.norm(b), name
+    d = t[:, None] - ref_y.numpy()
+    want = np.maximum(np.array(br.QUANTILES) * d, (np.array(br.QUANTILES) - 1) * d).sum() / n
+    assert abs(float(loss) - want) <= 1e-2 * want
+
+
 def test_training_reduces_loss(ht, finder):
     br = ht.bracket
     rng = np.random.default_rng(3)
