@@ -102,6 +102,33 @@ def test_extended_records_and_input_order(ht, finder):
         assert key(_merge(ht, finder, rec[perm])) == key(got)
 
 
+@pytest.mark.parametrize("n,lo,hi,span", [
+    (1, 2.0, 2.0, 10.0),          # one halo
+    (257, 40.0, 60.0, 100.0),     # every halo wider than 3/4 of a cell (one CTA each)
+    (3000, 1e-3, 1e-2, 100.0),    # every radius far below a cell (one thread each)
+    (4000, 0.01, 30.0, 60.0),     # both kinds, long kill chains, one cell row and many
+    (2500, 1.0, 3.0, 1e-3),       # all centres in one cell
+])
+@pytest.mark.parametrize("reduce", [False, True])
+def test_search_sizes_match_oracle(ht, finder, n, lo, hi, span, reduce):
+    rng = np.random.default_rng(n)
+    rec = rng.normal(0, 1, (n, 11)).astype(np.float32)
+    rec[:, :3] = rng.uniform(-span / 2, span, (n, 3))
+    rec[:, 6] = np.exp(rng.uniform(np.log(lo), np.log(hi + 1e-9), n))
+    got = _merge(ht, finder, rec, volume_reduction=reduce)
+    want = oc.merge_catalog(rec, volume_reduction=reduce)
+    if not reduce:
+        assert np.array_equal(got, want)
+        return
+    # the reduced radius is the cube root of r^3 minus sums of cap volumes in another order:
+    # FP64 sums of at most n caps, n 2^-53 of r^3, which a radius left with a share s of its
+    # volume carries as n 2^-53 / (3 s); s > 1e-6 leaves every radius within one ulp
+    assert got.shape == want.shape
+    other = [c for c in range(11) if c != 6]
+    assert np.array_equal(got[:, other], want[:, other])
+    assert _ulps(got[:, 6], want[:, 6]).max(initial=0) <= 1
+
+
 @pytest.mark.parametrize("ievol", [0, 1])
 def test_finalize_eulerian_matches_oracle(ht, finder, ievol):
     cat = ht.catalog
