@@ -36,10 +36,12 @@ struct ht_ctx {
     int2* d_cell = nullptr;        // (linear offset in the bound tile, char4 bits) per cell
     int cell_n1 = 0, cell_n2 = 0;  // tile dims d_cell was built for (0: none)
     // SPH window weights of kernel_strain (RadialShell.jl:225-274), which depend only on
-    // the two shell radii: row mp holds entries [wrow[mp], wrow[mp+1]) of (m1, weight)
+    // the two shell radii: row mp holds entries [wrow[mp], wrow[mp+1]), the weights of the
+    // consecutive shells from wfirst[mp] on
     int64_t nweights = 0;
     int32_t* d_wrow = nullptr;     // [nshells + 2]
-    double2* d_wpk = nullptr;      // per entry: (weight, m1 as a double), one 16-byte load
+    int32_t* d_wfirst = nullptr;   // [nshells + 2]
+    double* d_wts = nullptr;
     // result-neutral tunables (ht_ctx_tune)
     int tune_block_bits = 17;      // LEARNED order: spatial block of 2^bits cells
     int tune_pf_kz = 0;            // peak scan: planes per CTA (0: by grid size)

@@ -24,6 +24,7 @@
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
 #include <mutex>
 #include <string>
 
@@ -39,25 +40,25 @@ constexpr int kRec = 16;          // doubles per shell in the scratch profile
 constexpr int kSmallG = 8;        // lanes per peak
 constexpr int kPeaksPerItem = 32 / kSmallG;  // peaks per work item (one per group)
 
-// Scratch profile record, one per shell m (1-based); rows are 128-byte aligned, and the
-// twelve values the SPH window sums read (G, Gf, SR) fill the last 96 bytes, so that they
-// come in three 256-bit loads:
+// Scratch profile record, one per shell m (1-based); rows are 128-byte aligned, and the six
+// values of the strain's window sums start on a 32-byte boundary, so that they come in a
+// 256-bit and a 128-bit load:
 enum : int {
     P_FBAR = 0,
     P_CSRB = 1,   // running Srb numerator, RadialShell.jl:760-764
-    P_G = 4,      // 3: Gshell / rad
-    P_GF = 7,     // 3: Gshellf / rad
-    P_SR = 10,    // 6: (SR_LK + SR_KL) / rad for 11, 22, 33, 12, 13, 23
+    P_SR = 4,     // 6: (SR_LK + SR_KL) / rad for 11, 22, 33, 12, 13, 23
+    P_G = 10,     // 3: Gshell / rad
+    P_GF = 13,    // 3: Gshellf / rad
 };
-static_assert(P_GF == P_G + 3 && P_SR == P_G + 6 && P_SR + 6 == kRec && P_G % 4 == 0,
-              "G, Gf, SR: twelve contiguous doubles on a 32-byte boundary at the row's end");
+static_assert(P_SR % 4 == 0 && P_G == P_SR + 6 && P_GF == P_G + 3 && P_GF + 3 == kRec,
+              "SR, G, Gf: twelve contiguous doubles on a 32-byte boundary at the row's end");
 
-// Per-cell sums gathered for every shell.
-enum : int { V_F = 0, V_N = 1, V_G = 2, V_GF = 5, V_SR = 8, V_ROWS = 14 };
+// Per-cell sums gathered for every shell; from V_SR on in the order of a profile row.
+enum : int { V_F = 0, V_N = 1, V_SR = 2, V_G = 8, V_GF = 11, V_ROWS = 14 };
 
 // Shared-memory staging per group: [V_ROWS][G + 1] doubles for the shell sums (the last
 // column holds the totals), or [G + 1][kStepW] doubles for inward-walk steps.
-constexpr int kStepW = 14;
+constexpr int kStepW = 8;       // an inward step's strain, eigen trace and zvir
 __host__ __device__ constexpr int group_smem_doubles(int G) {
     return V_ROWS * (G + 1) > (G + 1) * kStepW ? V_ROWS * (G + 1) : (G + 1) * kStepW;
 }
@@ -86,8 +87,9 @@ struct WalkArgs {
     const double* irad;     // 1 / rad (0 for the centre shell)
     const double* irad3;    // 1 / rad^3
     int nshells;
-    const int32_t* wrow;   // SPH weight table: row mp = entries [wrow[mp], wrow[mp+1])
-    const double2* wpk;    // entry: (weight, m1)
+    const int32_t* wrow;   // SPH weight table: row mp = entries [wrow[mp], wrow[mp+1]),
+    const int32_t* wfirst; // of shells wfirst[mp], wfirst[mp] + 1, ...
+    const double* wts;
 
     const float* ct;
     int nx, ny, nz;
@@ -185,70 +187,104 @@ struct Group {
     }
 };
 
-struct Strain {
-    double E[6];   // 11, 22, 33, 12, 13, 23
-    double g[3];
-    double gf[3];
-};
-
-// kernel_strain (RadialShell.jl:225-274) centred on shell mp over the shells m1 of its
-// weight-table row with lo <= m1 <= hi, in FP64.  The row of mp > 1 lists the shells
-// with (rad[mp] - rad[m1])^2 < 4 and hRinteg(u0, u12) / (u12 - u0^2)^2 as weight; the
-// row of mp = 1 lists shells 2..U(1) with the atab4 weight 0.5 * W / rad[m1].  The
+// kernel_strain (RadialShell.jl:225-274) centred on shell mp over the shells m of its
+// weight-table row with lo <= m <= hi, in FP64.  The row of mp > 1 lists the shells
+// with (rad[mp] - rad[m])^2 < 4 and hRinteg(u0, u12) / (u12 - u0^2)^2 as weight; the
+// row of mp = 1 lists shells 2..U(1) with the atab4 weight 0.5 * W / rad[m].  The
 // weighted sums are scaled by wRnor / rad[mp] (mp > 1) or aRnor (mp = 1) at the end, in
 // the reference's order.
-// The twelve window values (G, Gf, SR) of a profile row in three 256-bit loads.  The rows
-// were written by the group's lanes before the post-processing began (the group synced
-// since), and this is the only access to them in the caller's loop.
-__device__ __forceinline__ void load_row12(const double* q, double (&r)[12]) {
-    const double* b = q + P_G;
+//
+// The strain (one lane per centre) and the gradients (one lane per component) are summed
+// apart: of the inward walk's steps only the last two need gradients, which halves what a
+// step reads.  A row's shells are consecutive, so that the loops have no exits and several
+// rows are in flight: a window is 20 to 70 rows long and its loads come from L2.
+
+// Six strain values (SR) of a profile row.  The rows were written by the group's lanes
+// before the post-processing began (the group synced since).
+__device__ __forceinline__ void load_sr(const double* row, double (&r)[6]) {
+    const double* b = row + P_SR;
     asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
                  : "=d"(r[0]), "=d"(r[1]), "=d"(r[2]), "=d"(r[3]) : "l"(b));
-    asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
-                 : "=d"(r[4]), "=d"(r[5]), "=d"(r[6]), "=d"(r[7]) : "l"(b + 4));
-    asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
-                 : "=d"(r[8]), "=d"(r[9]), "=d"(r[10]), "=d"(r[11]) : "l"(b + 8));
+    asm volatile("ld.global.v2.f64 {%0,%1}, [%2];" : "=d"(r[4]), "=d"(r[5]) : "l"(b + 4));
 }
 
+struct Window { int first, last; const double* w; };   // shells, and w[m] their weights
+__device__ __forceinline__ Window window_of(const int32_t* __restrict__ wrow,
+                                            const int32_t* __restrict__ wfirst,
+                                            const double* __restrict__ wts, int mp, int lo,
+                                            int hi) {
+    const int e0 = __ldg(wrow + mp), e1 = __ldg(wrow + mp + 1), f = __ldg(wfirst + mp);
+    return Window{max(f, lo), min(f + (e1 - e0) - 1, hi), wts + e0 - f};
+}
+
+struct Strain { double E[6]; };   // 11, 22, 33, 12, 13, 23
+
 __device__ __noinline__ Strain kernel_strain(const int32_t* __restrict__ wrow,
-                                             const double2* __restrict__ wpk,
+                                             const int32_t* __restrict__ wfirst,
+                                             const double* __restrict__ wts,
                                              const double* __restrict__ rad, double wRnor,
                                              double aRnor, const double* __restrict__ P,
                                              int mp, int lo, int hi) {
     Strain s;
 #pragma unroll
     for (int i = 0; i < 6; ++i) s.E[i] = 0.0;
+    const Window w = window_of(wrow, wfirst, wts, mp, lo, hi);
+    constexpr int kAhead = 4;
+    int m = w.first;
+    for (; m + kAhead - 1 <= w.last; m += kAhead) {
+        double hw[kAhead], r[kAhead][6];
 #pragma unroll
-    for (int i = 0; i < 3; ++i) { s.g[i] = 0.0; s.gf[i] = 0.0; }
-    const int e0 = __ldg(wrow + mp), e1 = __ldg(wrow + mp + 1);
-    for (int e = e0; e < e1; ++e) {
-        const double2 we = __ldg(wpk + e);
-        const int m1 = (int)we.y;
-        if (m1 > hi) break;
-        if (m1 < lo) continue;
-        const double wt = we.x;
-        const double hw = 0.5 * wt;
-        double r[12];
-        load_row12(P + (size_t)m1 * kRec, r);
-#pragma unroll
-        for (int L = 0; L < 3; ++L) {
-            s.g[L] += wt * r[L];
-            s.gf[L] += wt * r[3 + L];
+        for (int u = 0; u < kAhead; ++u) {
+            hw[u] = 0.5 * __ldg(w.w + m + u);
+            load_sr(P + (size_t)(m + u) * kRec, r[u]);
         }
 #pragma unroll
-        for (int i = 0; i < 6; ++i) s.E[i] -= hw * r[6 + i];
+        for (int u = 0; u < kAhead; ++u)
+#pragma unroll
+            for (int i = 0; i < 6; ++i) s.E[i] -= hw[u] * r[u][i];
+    }
+    for (; m <= w.last; ++m) {
+        const double hw = 0.5 * __ldg(w.w + m);
+        double r[6];
+        load_sr(P + (size_t)m * kRec, r);
+#pragma unroll
+        for (int i = 0; i < 6; ++i) s.E[i] -= hw * r[i];
     }
     const double scale = mp > 1 ? wRnor / rad[mp] : aRnor;
 #pragma unroll
     for (int i = 0; i < 6; ++i) s.E[i] *= scale;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) { s.g[i] *= scale; s.gf[i] *= scale; }
     return s;
 }
 
-// kernel_strain's central branch over shells lo..hi computed directly (used for the
-// gradient at the filter scale when mrf = 1, whose window starts at the centre shell:
-// its weight 0.5 * W(0) / 0 is infinite and the reference's gradient is NaN).
+// Component c of the gradient sums (0-2: G, 3-5: Gf).
+__device__ __noinline__ double kernel_gradient(const int32_t* __restrict__ wrow,
+                                               const int32_t* __restrict__ wfirst,
+                                               const double* __restrict__ wts,
+                                               const double* __restrict__ rad, double wRnor,
+                                               double aRnor, const double* P, int mp, int lo,
+                                               int hi, int c) {
+    const Window w = window_of(wrow, wfirst, wts, mp, lo, hi);
+    const double* q = P + P_G + c;
+    double s = 0.0;
+#pragma unroll 4
+    for (int m = w.first; m <= w.last; ++m) s += __ldg(w.w + m) * q[(size_t)m * kRec];
+    return s * (mp > 1 ? wRnor / rad[mp] : aRnor);
+}
+
+// The atab4 weight of the central branch at radius r1.
+__device__ __forceinline__ double central_weight(const double* __restrict__ akk, double r1) {
+    const double con = 100.0 * r1 * r1;
+    const double fl = floor(con);
+    const int icon = (int)fl;
+    const double diff = con - fl;
+    double aww = 0.0;
+    if (icon >= 0 && icon < 1100) aww = akk[icon] + diff * (akk[icon + 1] - akk[icon]);
+    return 0.5 * aww / r1;
+}
+
+// kernel_strain's central branch over shells lo..hi computed directly (used where the
+// window starts at the centre shell, as the gradient at the filter scale does when
+// mrf = 1: its weight 0.5 * W(0) / 0 is infinite and the reference's gradient is NaN).
 __device__ __noinline__ Strain kernel_strain_central(const double* __restrict__ rad,
                                                      const double* __restrict__ akk,
                                                      double aRnor,
@@ -257,33 +293,26 @@ __device__ __noinline__ Strain kernel_strain_central(const double* __restrict__ 
     Strain s;
 #pragma unroll
     for (int i = 0; i < 6; ++i) s.E[i] = 0.0;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) { s.g[i] = 0.0; s.gf[i] = 0.0; }
     for (int m1 = lo; m1 <= hi; ++m1) {
-        const double r1 = rad[m1];
-        const double con = 100.0 * r1 * r1;
-        const double fl = floor(con);
-        const int icon = (int)fl;
-        const double diff = con - fl;
-        double aww = 0.0;
-        if (icon >= 0 && icon < 1100) aww = akk[icon] + diff * (akk[icon + 1] - akk[icon]);
-        const double wt = 0.5 * aww / r1;
-        const double hw = 0.5 * wt;
-        double r[12];
-        load_row12(P + (size_t)m1 * kRec, r);
+        const double hw = 0.5 * central_weight(akk, rad[m1]);
+        double r[6];
+        load_sr(P + (size_t)m1 * kRec, r);
 #pragma unroll
-        for (int L = 0; L < 3; ++L) {
-            s.g[L] += wt * r[L];
-            s.gf[L] += wt * r[3 + L];
-        }
-#pragma unroll
-        for (int i = 0; i < 6; ++i) s.E[i] -= hw * r[6 + i];
+        for (int i = 0; i < 6; ++i) s.E[i] -= hw * r[i];
     }
 #pragma unroll
     for (int i = 0; i < 6; ++i) s.E[i] *= aRnor;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) { s.g[i] *= aRnor; s.gf[i] *= aRnor; }
     return s;
+}
+
+__device__ __noinline__ double kernel_gradient_central(const double* __restrict__ rad,
+                                                       const double* __restrict__ akk,
+                                                       double aRnor, const double* P, int lo,
+                                                       int hi, int c) {
+    double s = 0.0;
+    for (int m1 = lo; m1 <= hi; ++m1)
+        s += central_weight(akk, rad[m1]) * P[(size_t)m1 * kRec + P_G + c];
+    return s * aRnor;
 }
 
 // The walk's arguments stay in the kernel's parameter space (constant bank): functions
@@ -292,11 +321,15 @@ __device__ __noinline__ Strain kernel_strain_central(const double* __restrict__ 
 // local memory and read its fields from there.)
 __device__ __forceinline__ Strain strain_at(const WalkArgs& a, const double* P, int mp,
                                             int lo, int hi) {
-    return kernel_strain(a.wrow, a.wpk, a.rad, a.wRnor, a.aRnor, P, mp, lo, hi);
+    return kernel_strain(a.wrow, a.wfirst, a.wts, a.rad, a.wRnor, a.aRnor, P, mp, lo, hi);
 }
 __device__ __forceinline__ Strain strain_central(const WalkArgs& a, const double* P, int lo,
                                                  int hi) {
     return kernel_strain_central(a.rad, a.akk, a.aRnor, P, lo, hi);
+}
+__device__ __forceinline__ double gradient_at(const WalkArgs& a, const double* P, int mp,
+                                              int lo, int hi, int c) {
+    return kernel_gradient(a.wrow, a.wfirst, a.wts, a.rad, a.wRnor, a.aRnor, P, mp, lo, hi, c);
 }
 
 // Ascending eigenvalues of a symmetric 3x3 matrix by cyclic Jacobi rotations in FP64
@@ -416,8 +449,8 @@ __device__ __forceinline__ Shape shape_of(const double E[6]) {
     return s;
 }
 
-// zvir of one inward-walk step (RadialShell.jl:629-648): the step's strain, its
-// eigen trace (Frhoh) and zvir at shell mp.
+// One inward-walk step (RadialShell.jl:629-648): the step's strain, its eigen trace
+// (Frhoh) and zvir at shell mp.
 struct Step {
     Strain k;
     double trace;
@@ -690,7 +723,10 @@ __device__ __forceinline__ void process_peak(const WalkArgs& a, long long p, dou
         R[V_F * RP + t] = acc[0].value();
         R[V_N * RP + t] = (double)nin;
 #pragma unroll
-        for (int i = 0; i < 12; ++i) R[(V_G + i) * RP + t] = acc[1 + i].value();
+        for (int i = 0; i < 6; ++i) {   // acc: delta, G, Gf, SR
+            R[(V_G + i) * RP + t] = acc[1 + i].value();
+            R[(V_SR + i) * RP + t] = acc[7 + i].value();
+        }
         g.sync();
         for (int v = t; v < V_ROWS; v += G) {
             double sum = 0.0;
@@ -713,9 +749,9 @@ __device__ __forceinline__ void process_peak(const WalkArgs& a, long long p, dou
             double v;
             if (i == P_FBAR) v = Fbar_s;
             else if (i == P_CSRB) v = csrb;
-            else if (i < P_G) continue;   // unused
-            else if (i >= P_SR && i < P_SR + 3) v = (2.0 * R[(V_G + i - P_G) * RP + G]) * a.irad[s];
-            else v = R[(V_G + i - P_G) * RP + G] * a.irad[s];   // G, Gf, SR rows in order
+            else if (i < P_SR) continue;   // unused
+            else if (i < P_SR + 3) v = (2.0 * R[(V_SR + i - P_SR) * RP + G]) * a.irad[s];
+            else v = R[(V_SR + i - P_SR) * RP + G] * a.irad[s];   // SR, G, Gf rows in order
             q[i] = v;
         }
         g.sync();
@@ -740,12 +776,11 @@ __device__ __forceinline__ void process_peak(const WalkArgs& a, long long p, dou
     // ------------------------------------------------------ post-processing ----
     // gradient at the filter scale (RadialShell.jl:466-482); when mrf = 1 the window
     // starts at the centre shell
-    double gradpkrf[3];
-    {
-        const Strain k = bd.mrf > 1 ? strain_at(a, P, bd.mrf, 1, bd.need_rf)
-                                    : strain_central(a, P, 1, bd.need_rf);
-        gradpkrf[0] = k.g[0]; gradpkrf[1] = k.g[1]; gradpkrf[2] = k.g[2];
-    }
+    double gradpkrf = 0.0;   // component t
+    if (t < 3)
+        gradpkrf = bd.mrf > 1 ? gradient_at(a, P, bd.mrf, 1, bd.need_rf, t)
+                              : kernel_gradient_central(a.rad, a.akk, a.aRnor, P, 1,
+                                                        bd.need_rf, t);
 
     // crossing (RadialShell.jl:485-526)
     int m0 = bd.m0_init;
@@ -783,10 +818,8 @@ __device__ __forceinline__ void process_peak(const WalkArgs& a, long long p, dou
             const Step st = eval_step(a, P, m0 - u, m, u == 0);
 #pragma unroll
             for (int i = 0; i < 6; ++i) row[i] = st.k.E[i];
-#pragma unroll
-            for (int i = 0; i < 3; ++i) { row[6 + i] = st.k.g[i]; row[9 + i] = st.k.gf[i]; }
-            row[12] = st.trace;
-            row[13] = st.zvir;
+            row[6] = st.trace;
+            row[7] = st.zvir;
             hit = st.zvir >= ZZon;
         }
         const unsigned bal = g.ballot(hit);
@@ -798,7 +831,7 @@ __device__ __forceinline__ void process_peak(const WalkArgs& a, long long p, dou
             prow = l > 0 ? l - 1 : G;
             break;
         }
-        for (int i = t; i < 14; i += G) R[G * kStepW + i] = R[(G - 1) * kStepW + i];
+        for (int i = t; i < kStepW; i += G) R[G * kStepW + i] = R[(G - 1) * kStepW + i];
         g.sync();
     }
     if (tstar < 0 || (tstar == 0 && m0 == 1)) {
@@ -814,8 +847,8 @@ __device__ __forceinline__ void process_peak(const WalkArgs& a, long long p, dou
     const double* Pr = R + prow * kStepW;   // the step before it ("prev")
 
     const int m0f = m0 - tstar + 1;   // collapse at shell mp* = m0f - 1
-    const double zvir1p = Lr[13];
-    const double zvir1 = tstar == 0 ? -1.0 : Pr[13];
+    const double zvir1p = Lr[7];
+    const double zvir1 = tstar == 0 ? -1.0 : Pr[7];
     const double dZ = zvir1p - zvir1;
     const double rp = rad[m0f - 1], rm = rad[m0f];
     double RTHL;
@@ -835,23 +868,24 @@ __device__ __forceinline__ void process_peak(const WalkArgs& a, long long p, dou
     const double rad3p = rp * rp * rp, rad3 = rm * rm * rm, drad3 = rad3 - rad3p;
     const double Fb_m = P[(size_t)m0f * kRec + P_FBAR];
     const double Fb_p = P[(size_t)(m0f - 1) * kRec + P_FBAR];
-    double Fbarx, smat[6], gpk[3], gpkf[3];
+    double Fbarx, smat[6], gpk = 0.0;
+    // gradient component t (0-2: gradpk, 3-5: gradpkf) at the step before the collapse and,
+    // where the results are interpolated, at the collapse
+    const double gPrev = t < 6 ? gradient_at(a, P, tstar == 0 ? m0 : m0f, 1, m, t) : 0.0;
     if (zvir1 > 0.0 && drad3 != 0.0) {
         const double frac = (RTHL3 - rad3p) / drad3;
         Fbarx = Fb_p + frac * (Fb_m - Fb_p);
 #pragma unroll
         for (int i = 0; i < 6; ++i) smat[i] = Lr[i] + frac * (Pr[i] - Lr[i]);
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            gpk[i] = Lr[6 + i] + frac * (Pr[6 + i] - Lr[6 + i]);
-            gpkf[i] = Lr[9 + i] + frac * (Pr[9 + i] - Lr[9 + i]);
+        if (t < 6) {
+            const double gLast = gradient_at(a, P, m0f - 1, 1, m, t);
+            gpk = gLast + frac * (gPrev - gLast);
         }
     } else {
         Fbarx = Fb_p;
 #pragma unroll
         for (int i = 0; i < 6; ++i) smat[i] = Lr[i];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) { gpk[i] = Pr[6 + i]; gpkf[i] = Pr[9 + i]; }
+        gpk = gPrev;
     }
     // normalize_strain + eigen (RadialShell.jl:730-734)
     const double tr = smat[0] + smat[1] + smat[2];
@@ -863,7 +897,7 @@ __device__ __forceinline__ void process_peak(const WalkArgs& a, long long p, dou
     const Shape fin = shape_of(smat);
     // strain_final (RadialShell.jl:736, guarded as ShellAnalysisGPU.jl:459)
     double sfin[6];
-    const double Frhoh = Lr[12];
+    const double Frhoh = Lr[6];
     if (a.conv == HT_CONV_GPU && Frhoh == 0.0) {
 #pragma unroll
         for (int i = 0; i < 6; ++i) sfin[i] = Lr[i];
@@ -1034,10 +1068,11 @@ __device__ __forceinline__ void process_peak(const WalkArgs& a, long long p, dou
     if (t < 3) {
         o.Sbar[3 * p + t] = (float)Sb[t];
         o.Sbar2[3 * p + t] = (float)Sb2[t];
-        o.gradpk[3 * p + t] = (float)gpk[t];
-        o.gradpkf[3 * p + t] = (float)gpkf[t];
-        o.gradpkrf[3 * p + t] = (float)gradpkrf[t];
+        o.gradpk[3 * p + t] = (float)gpk;
+        o.gradpkrf[3 * p + t] = (float)gradpkrf;
         o.eigs[3 * p + t] = (float)fin.lam[t];
+    } else if (t < 6) {
+        o.gradpkf[3 * p + t - 3] = (float)gpk;
     }
 }
 
@@ -1095,13 +1130,36 @@ __global__ void __launch_bounds__(kThreads, 3) walk_kernel(const WalkArgs a) {
     if (threadIdx.x < HT_REJECT_COUNT && a.reject && rej[threadIdx.x])
         atomicAdd(a.reject + threadIdx.x, (unsigned long long)rej[threadIdx.x]);
 }
-// Processing order for BATCHED mode: key = Morton code of the 0-based (i, j, k), 20 bits
-// per axis; in LEARNED mode coarse spatial blocks of 2^block_bits cells (a Morton prefix)
-// and, inside a block, the predicted walk cost (descending).  Peaks consecutive in this
-// order sit close together in the tile, so the warps walking them at the same time
-// gather largely the same cell records, which then come from L2; in LEARNED mode the four
-// peaks of a warp also walk similar distances.  The order changes no result (outputs are
-// indexed by peak).
+// Processing order for BATCHED mode: key = Morton code of the 0-based (i, j, k); in LEARNED
+// mode coarse spatial blocks of 2^block_bits cells (a Morton prefix) and, inside a block, the
+// predicted walk cost (descending).  Peaks consecutive in this order sit close together in
+// the tile, so the warps walking them at the same time gather largely the same cell records,
+// which then come from L2; in LEARNED mode the four peaks of a warp also walk similar
+// distances.  Walks past kLongWalk cells go first, in the same order among themselves: one
+// of them is a chain of loads up to milliseconds long, and those that came last kept a few
+// warps busy after the others were done (43 % of the SM cycles of a 140,000-peak walk of a
+// 320^3 tile were idle; the walk went from 5.13 to 4.75 ms and that of 40,000 peaks of a
+// 200^3 tile from 1.96 to 1.71; a line at 10 cells was no better, and cost the 2.2 M peaks
+// of a 620^3 tile 2 % in locality, 16 cells nothing).  The order changes no result (outputs are indexed by
+// peak).
+constexpr float kLongWalk = 16.f;
+// The keys are 32 bits wide (four passes of the sort): a long-walk bit over KeyBits.place
+// bits of the Morton code and, in LEARNED mode, kCostBits of cost in 1/16 cells.
+constexpr int kCostBits = 12;
+struct KeyBits {
+    int shift, place;    // Morton bits dropped and kept
+    int total;
+};
+static KeyBits key_bits(int n, int block_bits, bool cost) {
+    int nb = 1;
+    while (nb < 20 && (1 << nb) < n) ++nb;
+    const int room = 31 - (cost ? kCostBits : 0);
+    KeyBits k;
+    k.shift = std::max(cost ? std::min(block_bits, 3 * nb) : 0, 3 * nb - room);
+    k.place = 3 * nb - k.shift;
+    k.total = k.place + 1 + (cost ? kCostBits : 0);
+    return k;
+}
 __device__ __forceinline__ unsigned long long spread3(unsigned v) {
     unsigned long long x = v & 0xfffffu;
     x = (x | x << 32) & 0x1f00000000ffffULL;
@@ -1113,7 +1171,8 @@ __device__ __forceinline__ unsigned long long spread3(unsigned v) {
 }
 
 __global__ void __launch_bounds__(256) order_key_kernel(const WalkArgs a,
-                                                        unsigned long long* __restrict__ keys,
+                                                        KeyBits kb,
+                                                        uint32_t* __restrict__ keys,
                                                         int32_t* __restrict__ idx,
                                                         int4* __restrict__ bounds,
                                                         const float* __restrict__ cost) {
@@ -1125,17 +1184,17 @@ __global__ void __launch_bounds__(256) order_key_kernel(const WalkArgs a,
     const unsigned i = (unsigned)max(a.pi[p] - 1, 0), j = (unsigned)max(a.pj[p] - 1, 0),
                    k = (unsigned)max(a.pk[p] - 1, 0);
     const unsigned long long mort = spread3(i) | (spread3(j) << 1) | (spread3(k) << 2);
+    const uint32_t place = (uint32_t)(mort >> kb.shift) & (uint32_t)((1ull << kb.place) - 1);
+    float reach = (float)a.rad[b.m0_init] + 2.f;   // at least this far
+    uint32_t key = place;
     if (cost) {
-        // learned order: coarse spatial blocks of 2^block_bits cells (Morton prefix, keeps
-        // the L2 locality), then descending predicted cost (1/16-cell steps, 24 bits)
         float c = cost[p];
         c = c == c ? fminf(fmaxf(c, 0.f), 1.0e6f) : 0.f;
-        const unsigned long long q = min((unsigned long long)(c * 16.f), 0xFFFFFFull);
-        const unsigned long long blk = (mort >> a.block_bits) & ((1ull << 38) - 1);
-        keys[p] = (blk << 24) | (0xFFFFFFull - q);
-    } else {
-        keys[p] = mort;
+        reach = c;
+        const uint32_t top = (1u << kCostBits) - 1;
+        key = (place << kCostBits) | (top - min((uint32_t)(c * 16.f), top));
     }
+    keys[p] = key | (reach > kLongWalk ? 0u : 1u << (kb.total - 1));
     idx[p] = (int32_t)p;
 }
 
@@ -1224,7 +1283,7 @@ static void fill_args(WalkArgs& a, const ht_ctx* ctx, const ht_fields& f, const 
     a.irad = ctx->d_irad; a.irad3 = ctx->d_irad3;
     a.cell = nullptr; a.nhunt = ctx->nhunt;
     for (int jj = 0; jj < 10; ++jj) a.zh_frac[jj] = cbrt(jj / 9.0 * 0.5 + 0.5);
-    a.wrow = ctx->d_wrow; a.wpk = ctx->d_wpk;
+    a.wrow = ctx->d_wrow; a.wfirst = ctx->d_wfirst; a.wts = ctx->d_wts;
     a.ct = ctx->d_ct; a.nx = ctx->nx; a.ny = ctx->ny; a.nz = ctx->nz;
     a.X1 = ctx->X1; a.X2 = ctx->X2; a.Y1 = ctx->Y1; a.Y2 = ctx->Y2; a.Z1 = ctx->Z1;
     a.Z2 = ctx->Z2; a.out_val = ctx->out_val; a.akk = ctx->d_akk;
@@ -1311,32 +1370,32 @@ int ht_launch_walk(ht_ctx* ctx, const ht_peak_batch* b, double alatt, double rma
         size_t temp = 0;
         if (sort)
             HT_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp,
-                                                        (unsigned long long*)nullptr,
-                                                        (unsigned long long*)nullptr,
+                                                        (uint32_t*)nullptr, (uint32_t*)nullptr,
                                                         (int32_t*)nullptr, (int32_t*)nullptr, np,
-                                                        0, 63, st),
+                                                        0, 32, st),
                         "radix sort size query");
         const size_t bb = ((size_t)np * 16 + 255) / 256 * 256;
-        const size_t kb = sort ? ((size_t)np * 8 + 255) / 256 * 256 : 0;
+        const size_t kb = sort ? ((size_t)np * 4 + 255) / 256 * 256 : 0;
         const size_t ib = sort ? ((size_t)np * 4 + 255) / 256 * 256 : 0;
         rc = ht_grow(&ctx->d_order_ws, &ctx->order_ws_bytes, bb + 2 * kb + 2 * ib + temp,
                      "peak-order workspace");
         if (rc != HT_OK) return rc;
         char* w = (char*)ctx->d_order_ws;
         int4* bounds = (int4*)w;
-        unsigned long long* k_in = sort ? (unsigned long long*)(w + bb) : nullptr;
-        unsigned long long* k_out = sort ? (unsigned long long*)(w + bb + kb) : nullptr;
+        uint32_t* k_in = sort ? (uint32_t*)(w + bb) : nullptr;
+        uint32_t* k_out = sort ? (uint32_t*)(w + bb + kb) : nullptr;
         int32_t* v_in = sort ? (int32_t*)(w + bb + 2 * kb) : nullptr;
         int32_t* v_out = sort ? (int32_t*)(w + bb + 2 * kb + ib) : nullptr;
         void* tmp = w + bb + 2 * kb + 2 * ib;
         const float* cost = mode == HT_MODE_LEARNED ? b->cost : nullptr;
-        order_key_kernel<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(a, k_in, v_in, bounds,
+        const KeyBits bits = key_bits(std::max({a.n1, a.n2, a.n3}), a.block_bits, cost != nullptr);
+        order_key_kernel<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(a, bits, k_in, v_in, bounds,
                                                                         cost);
         HT_CUDA_TRY(cudaGetLastError(), "order_key_kernel launch");
         nk = 1;
         if (sort) {
             HT_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, temp, k_in, k_out, v_in, v_out,
-                                                        np, 0, 63, st),
+                                                        np, 0, bits.total, st),
                         "radix sort of the peak order");
             a.order = v_out;
             nk += 3;   // the radix sort's passes (approximate count)
