@@ -53,6 +53,16 @@ __device__ __forceinline__ double dist3(double ax, double ay, double az, double 
     return __dsqrt_rn(dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz)));
 }
 
+// dist3(a, b) < r for r > 0.  The squares decide it beyond 1e-12 of the line (their roundings
+// and the root's move it by a few 1e-16); on the line the rounded root does.
+__device__ __forceinline__ bool within(const float4& a, const float4& b, double r) {
+    const double dx = (double)b.x - a.x, dy = (double)b.y - a.y, dz = (double)b.z - a.z;
+    const double s = dx * dx + dy * dy + dz * dz, rr = r * r;
+    if (s < rr * (1.0 - 1e-12) && rr < 1e300) return true;
+    if (s > rr * (1.0 + 1e-12) && s < 1e300) return false;
+    return dist3(a.x, a.y, a.z, b.x, b.y, b.z) < r;
+}
+
 __global__ void extract_kernel(const float* __restrict__ rec, long long n, int width,
                                float* __restrict__ x, float* __restrict__ y,
                                float* __restrict__ z, float* __restrict__ r,
@@ -119,6 +129,7 @@ enum : uint8_t { kUndecided = 0, kAlive = 1, kDead = 2 };
 struct Nbr {
     const float4* xyzr;
     const int32_t* rank;
+    const int32_t* open;       // the rank while the halo is undecided, then -1
     const int32_t* cstart;     // nc^3 + 1
     Grid g;
     // A halo whose radius exceeds `big` is searched by a whole CTA instead of one thread:
@@ -161,12 +172,13 @@ __device__ __forceinline__ void for_neighbours(const Nbr& nb, const Box& b, F&& 
 // cell order: attributes, the inverse of `list` (ranks by cell), and how many ranks are big
 __global__ void cell_order_kernel(const int32_t* __restrict__ list, long long n,
                                   const float4* __restrict__ by_rank, float big,
-                                  float4* __restrict__ xyzr, int32_t* __restrict__ at,
-                                  int32_t* __restrict__ nbig) {
+                                  float4* __restrict__ xyzr, int32_t* __restrict__ open,
+                                  int32_t* __restrict__ at, int32_t* __restrict__ nbig) {
     const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const int q = list[s];
     xyzr[s] = by_rank[q];
+    open[s] = q;
     at[q] = (int32_t)s;
     // ranks are in decreasing radius: the last big one knows the count
     if (by_rank[s].w > big && (s == n - 1 || !(by_rank[s + 1].w > big))) *nbig = (int32_t)s + 1;
@@ -195,12 +207,13 @@ __global__ void __launch_bounds__(kCta ? 128 : 256) push_kernel(
         const float4 v = nb.xyzr[s];
         if (!kCta && v.w > nb.big) return;
         const double rq = v.w;
+        if (!(rq > 0.0)) return;   // covers nothing
         const int rank = nb.rank[s];
         uint8_t* mark = fresh ? killed : blocked;
         for_neighbours<kCta>(nb, box_of(nb.g, v, rq), [&](int p) {
-            if (status[p] != kUndecided || nb.rank[p] <= rank) return;
-            const float4 w = nb.xyzr[p];
-            if (dist3(v.x, v.y, v.z, w.x, w.y, w.z) < rq) mark[p] = 1;
+            if (__ldg(nb.open + p) <= rank) return;   // decided, or earlier in the order
+            const float4 w = __ldg(nb.xyzr + p);
+            if (within(v, w, rq)) mark[p] = 1;
         });
     };
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -215,16 +228,18 @@ __global__ void __launch_bounds__(kCta ? 128 : 256) push_kernel(
 __global__ void __launch_bounds__(256) decide_kernel(
     long long n, uint8_t* __restrict__ status, int32_t* __restrict__ alive_round, int round,
     uint8_t* __restrict__ blocked, const uint8_t* __restrict__ killed,
-    const unsigned long long* __restrict__ before, unsigned long long* __restrict__ left) {
+    int32_t* __restrict__ open_rank, const unsigned long long* __restrict__ before, unsigned long long* __restrict__ left) {
     if (before && *before == 0) return;   // and *left stays 0
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     bool open = false;
     if (p < n && status[p] == kUndecided) {
         if (killed[p]) {
             status[p] = kDead;
+            open_rank[p] = -1;
         } else if (!blocked[p]) {
             status[p] = kAlive;
             alive_round[p] = round;
+            open_rank[p] = -1;
         } else {
             blocked[p] = 0;   // for the next round (a killed halo is decided for good)
             open = true;
@@ -446,7 +461,7 @@ extern "C" HT_API int ht_merge_halos(ht_ctx* ctx, const float* d_records, int64_
     tb = std::max(tb, t1);
     float *x, *y, *z, *r, *new_r, *ext;
     uint32_t *k0, *k1, *c0, *c1;
-    int32_t *i0, *i1, *l0, *l1, *alive_round, *sidx, *at;
+    int32_t *i0, *i1, *l0, *l1, *alive_round, *sidx, *at, *open_rank;
     float4 *xyzr, *cxyzr;
     uint8_t* flags;
     double* dV;
@@ -468,6 +483,7 @@ extern "C" HT_API int ht_merge_halos(ht_ctx* ctx, const float* d_records, int64_
         xyzr = carve<float4>(cur, n);
         cxyzr = carve<float4>(cur, n);
         at = carve<int32_t>(cur, n);
+        open_rank = carve<int32_t>(cur, n);
         c0 = carve<uint32_t>(cur, n);
         c1 = carve<uint32_t>(cur, n);
         l0 = carve<int32_t>(cur, n);
@@ -558,9 +574,9 @@ extern "C" HT_API int ht_merge_halos(ht_ctx* ctx, const float* d_records, int64_
                     "cub::DeviceRadixSort::SortPairs (cells)");
     }
     const float big = (float)(0.75 * g.cs);
-    Nbr nb{cxyzr, l1, cstart, g, big, nbig, at};
+    Nbr nb{cxyzr, l1, open_rank, cstart, g, big, nbig, at};
     HT_CUDA_TRY(cudaMemsetAsync(nbig, 0, sizeof(int32_t), st), "big count reset");
-    cell_order_kernel<<<blocks, 256, 0, st>>>(l1, n, xyzr, big, cxyzr, at, nbig);
+    cell_order_kernel<<<blocks, 256, 0, st>>>(l1, n, xyzr, big, cxyzr, open_rank, at, nbig);
     HT_CUDA_TRY(cudaGetLastError(), "cell_order_kernel launch");
     const unsigned big_ctas = (unsigned)std::min<long long>(n, 16LL * ctx->num_sms);
     // ---- exclusion rounds ----
@@ -581,7 +597,7 @@ extern "C" HT_API int ht_merge_halos(ht_ctx* ctx, const float* d_records, int64_
             push_kernel<false><<<blocks, 256, 0, st>>>(nb, n, status, alive_round, rounds, before,
                                                        blocked, killed);
             decide_kernel<<<blocks, 256, 0, st>>>(n, status, alive_round, rounds, blocked, killed,
-                                                  before, now + k);
+                                                  open_rank, before, now + k);
             HT_CUDA_TRY(cudaGetLastError(), "exclusion round launch");
         }
         unsigned long long h_left = 0;
