@@ -53,15 +53,9 @@ enum : int {
 static_assert(P_SR % 4 == 0 && P_G == P_SR + 6 && P_GF == P_G + 3 && P_GF + 3 == kRec,
               "SR, G, Gf: twelve contiguous doubles on a 32-byte boundary at the row's end");
 
-// Per-cell sums gathered for every shell; from V_SR on in the order of a profile row.
-enum : int { V_F = 0, V_N = 1, V_SR = 2, V_G = 8, V_GF = 11, V_ROWS = 14 };
-
-// Shared-memory staging per group: [V_ROWS][G + 1] doubles for the shell sums (the last
-// column holds the totals), or [G + 1][kStepW] doubles for inward-walk steps.
+// Shared-memory staging per group: [G + 1][kStepW] doubles for inward-walk steps.
 constexpr int kStepW = 8;       // an inward step's strain, eigen trace and zvir
-__host__ __device__ constexpr int group_smem_doubles(int G) {
-    return V_ROWS * (G + 1) > (G + 1) * kStepW ? V_ROWS * (G + 1) : (G + 1) * kStepW;
-}
+__host__ __device__ constexpr int group_smem_doubles(int G) { return (G + 1) * kStepW; }
 constexpr int kWarpSmemDoubles = kPeaksPerItem * group_smem_doubles(kSmallG);
 
 struct WalkArgs {
@@ -215,6 +209,22 @@ __device__ __forceinline__ Window window_of(const int32_t* __restrict__ wrow,
                                             int hi) {
     const int e0 = __ldg(wrow + mp), e1 = __ldg(wrow + mp + 1), f = __ldg(wfirst + mp);
     return Window{max(f, lo), min(f + (e1 - e0) - 1, hi), wts + e0 - f};
+}
+
+// v[i] summed over the 8 lanes of a group, lane t ending with the sums 2 t and 2 t + 1: at
+// each of three exchanges a lane keeps half of its values and hands the other half to its
+// partner (14 exchanges of 64 bits for 16 values).
+__device__ __forceinline__ void reduce_scatter(const Group& g, double (&v)[16]) {
+    static_assert(kSmallG == 8, "three exchanges");
+#pragma unroll
+    for (int half = 8; half >= 2; half >>= 1) {
+        const bool hi = (g.t & (half >> 1)) != 0;
+#pragma unroll
+        for (int i = 0; i < half; ++i) {
+            const double give = hi ? v[i] : v[i + half], keep = hi ? v[i + half] : v[i];
+            v[i] = keep + __shfl_xor_sync(g.mask, give, half >> 1, kSmallG);
+        }
+    }
 }
 
 struct Strain { double E[6]; };   // 11, 22, 33, 12, 13, 23
@@ -660,7 +670,7 @@ template <bool PACKED>
 __device__ __forceinline__ void process_peak(const WalkArgs& a, long long p, double* __restrict__ P,
                              double* __restrict__ R, const Group& g, unsigned* rej) {
     const double* rad = a.rad;
-    const int G = g.G, t = g.t, RP = G + 1;
+    const int G = g.G, t = g.t;
     const int ci = a.pi[p], cj = a.pj[p], ck = a.pk[p];
     const double ZZon = (double)a.ZZon[p];
     const double fcrit = (double)a.fcrit[p];
@@ -719,42 +729,37 @@ __device__ __forceinline__ void process_peak(const WalkArgs& a, long long p, dou
             acc[11].add_prod(e0, d2); acc[11].add_prod(e2, d0);
             acc[12].add_prod(e1, d2); acc[12].add_prod(e2, d1);
         });
-        // combine the lanes in FP64, lanes 0..G-1 in order (deterministic)
-        R[V_F * RP + t] = acc[0].value();
-        R[V_N * RP + t] = (double)nin;
+        // combine the lanes in FP64, in the order of the profile row: delta and the count in
+        // the places of Fbar and the Srb numerator, then SR, G, Gf.   (By exchange: through
+        // shared memory, 14 stores and 16 loads of 64 bits per lane with conflicts, it took a
+        // third of the walk's L1 wavefronts and two barriers.)
+        double v[16];
+        v[0] = acc[0].value();
+        v[1] = (double)nin;
+        v[2] = v[3] = 0.0;
 #pragma unroll
         for (int i = 0; i < 6; ++i) {   // acc: delta, G, Gf, SR
-            R[(V_G + i) * RP + t] = acc[1 + i].value();
-            R[(V_SR + i) * RP + t] = acc[7 + i].value();
+            v[P_SR + i] = acc[7 + i].value();
+            v[P_G + i] = acc[1 + i].value();
         }
-        g.sync();
-        for (int v = t; v < V_ROWS; v += G) {
-            double sum = 0.0;
-            for (int u = 0; u < G; ++u) sum += R[v * RP + u];
-            R[v * RP + G] = sum;
-        }
-        g.sync();
+        reduce_scatter(g, v);           // lane t: row values 2 t, 2 t + 1 in v[0], v[1]
+        const double Fs = __shfl_sync(g.mask, v[0], 0, kSmallG);
+        const double ns = __shfl_sync(g.mask, v[1], 0, kSmallG);
         // finalise shell s (ShellAnalysisGPU.jl:197-228)
-        const double Fs = R[V_F * RP + G];
-        const double ns = R[V_N * RP + G];
         const double rs = rad[s];
         const double dF = ns > 0.0 ? Fs / ns : 0.0;
         const double r3p = radp * radp * radp, r3 = rs * rs * rs;
         const double Fbar_s = (r3p * Fbarp + 0.5 * (dFbarp + dF) * (r3 - r3p)) * a.irad3[s];
         const double r5 = rs * rs * rs * rs * rs;
         csrb += 0.5 * (Fbarp + Fbar_s) * (r5 - rad5p);
-        double* q = P + (size_t)s * kRec;
         if (!HT_INDEX_OK(a.status, s, a.nshells + 2)) break;
-        for (int i = t; i < kRec; i += G) {
-            double v;
-            if (i == P_FBAR) v = Fbar_s;
-            else if (i == P_CSRB) v = csrb;
-            else if (i < P_SR) continue;   // unused
-            else if (i < P_SR + 3) v = (2.0 * R[(V_SR + i - P_SR) * RP + G]) * a.irad[s];
-            else v = R[(V_SR + i - P_SR) * RP + G] * a.irad[s];   // SR, G, Gf rows in order
-            q[i] = v;
+        {
+            static_assert(P_FBAR == 0 && P_CSRB == 1 && P_SR == 4, "a row's places");
+            const double ir = a.irad[s];
+            const double x = t == 0 ? Fbar_s : (t == 2 || t == 3 ? 2.0 * v[0] : v[0]) * ir;
+            const double y = t == 0 ? csrb : (t == 2 ? 2.0 * v[1] : v[1]) * ir;
+            *reinterpret_cast<double2*>(P + (size_t)s * kRec + 2 * t) = make_double2(x, y);
         }
-        g.sync();
         cells_in += ns;
         Fbarp = Fbar_s; dFbarp = dF; radp = rs; rad5p = r5;
         s_end = s;
@@ -772,6 +777,7 @@ __device__ __forceinline__ void process_peak(const WalkArgs& a, long long p, dou
         atomicAdd(a.stats + 1, (unsigned long long)s_end);
     }
     write_walk_shells(a, p, g, s_end);
+    g.sync();   // the profile's rows, for every lane of the group
 
     // ------------------------------------------------------ post-processing ----
     // gradient at the filter scale (RadialShell.jl:466-482); when mrf = 1 the window
@@ -1095,9 +1101,14 @@ __device__ __forceinline__ void process_item(const WalkArgs& a, long long item, 
     __syncwarp();
 }
 
-// 3 blocks per SM: 80 registers; the few spills cost less than the lost occupancy.
-template <bool PACKED>
-__global__ void __launch_bounds__(kThreads, 3) walk_kernel(const WalkArgs a) {
+// BPSM blocks per SM.  With 3 (80 registers, some spills) the walk of 2.2 M peaks of a 620^3
+// tile takes 31.9 ms, with 2 (128 registers, no spills) 32.4; but small batches end on the
+// chains of their longest walks, which 2 make shorter: 140,000 peaks 4.31 against 4.69 ms,
+// 40,000 peaks 1.57 against 1.69, 200 peaks 0.33 against 0.39.  Below kFewPeaks the packed
+// walk takes 2.
+constexpr long long kFewPeaks = 500000;
+template <bool PACKED, int BPSM>
+__global__ void __launch_bounds__(kThreads, BPSM) walk_kernel(const WalkArgs a) {
     extern __shared__ double smem[];
     __shared__ unsigned rej[HT_REJECT_COUNT];   // the block's reject counts
     if (threadIdx.x < HT_REJECT_COUNT) rej[threadIdx.x] = 0u;
@@ -1140,7 +1151,7 @@ __global__ void __launch_bounds__(kThreads, 3) walk_kernel(const WalkArgs a) {
 // warps busy after the others were done (43 % of the SM cycles of a 140,000-peak walk of a
 // 320^3 tile were idle; the walk went from 5.13 to 4.75 ms and that of 40,000 peaks of a
 // 200^3 tile from 1.96 to 1.71; a line at 10 cells was no better, and cost the 2.2 M peaks
-// of a 620^3 tile 2 % in locality, 16 cells nothing).  The order changes no result (outputs are indexed by
+// of a 620^3 tile 2 % in locality).  The order changes no result (outputs are indexed by
 // peak).
 constexpr float kLongWalk = 16.f;
 // The keys are 32 bits wide (four passes of the sort): a long-walk bit over KeyBits.place
@@ -1305,14 +1316,14 @@ static size_t walk_smem_bytes() {
     return (size_t)kWarpsPerBlock * kWarpSmemDoubles * sizeof(double);
 }
 
-template <bool PACKED>
+template <bool PACKED, int BPSM>
 static int walk_blocks_per_sm(int* bpsm) {
     const size_t smem = walk_smem_bytes();
-    cudaError_t e = cudaFuncSetAttribute(walk_kernel<PACKED>,
+    cudaError_t e = cudaFuncSetAttribute(walk_kernel<PACKED, BPSM>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpsm, walk_kernel<PACKED>, kThreads,
-                                                          smem);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpsm, walk_kernel<PACKED, BPSM>,
+                                                          kThreads, smem);
     if (e != cudaSuccess) return ht_cuda_fail(e, "walk_kernel occupancy query");
     if (*bpsm < 1) *bpsm = 1;
     return HT_OK;
@@ -1323,7 +1334,9 @@ int ht_launch_walk(ht_ctx* ctx, const ht_peak_batch* b, double alatt, double rma
                    const ht_results* out, cudaStream_t st) {
     const bool packed = mode != HT_MODE_PLAIN;   // BATCHED and LEARNED
     int bpsm = 0;
-    int rc = packed ? walk_blocks_per_sm<true>(&bpsm) : walk_blocks_per_sm<false>(&bpsm);
+    const bool few = b->npeaks < kFewPeaks;
+    int rc = !packed ? walk_blocks_per_sm<false, 3>(&bpsm)
+             : few   ? walk_blocks_per_sm<true, 2>(&bpsm) : walk_blocks_per_sm<true, 3>(&bpsm);
     if (rc != HT_OK) return rc;
     if (ctx->tune_walk_bpsm > 0 && ctx->tune_walk_bpsm < bpsm) bpsm = ctx->tune_walk_bpsm;
     long long blocks = (long long)ctx->num_sms * bpsm;
@@ -1406,8 +1419,9 @@ int ht_launch_walk(ht_ctx* ctx, const ht_peak_batch* b, double alatt, double rma
     HT_CUDA_TRY(cudaMemsetAsync(ctx->d_stats, 0, 2 * sizeof(unsigned long long), st),
                 "stats reset");
     const size_t smem = walk_smem_bytes();
-    if (packed) walk_kernel<true><<<(unsigned)blocks, kThreads, smem, st>>>(a);
-    else walk_kernel<false><<<(unsigned)blocks, kThreads, smem, st>>>(a);
+    if (!packed) walk_kernel<false, 3><<<(unsigned)blocks, kThreads, smem, st>>>(a);
+    else if (few) walk_kernel<true, 2><<<(unsigned)blocks, kThreads, smem, st>>>(a);
+    else walk_kernel<true, 3><<<(unsigned)blocks, kThreads, smem, st>>>(a);
     HT_CUDA_TRY(cudaGetLastError(), "walk_kernel launch");
     ctx->last_kernels = 1 + nk;
     return HT_OK;
@@ -1495,7 +1509,7 @@ extern "C" HT_API int ht_shell_analyse_static(ht_ctx* ctx, const ht_fields* f,
     int rc = static_scratch_address(ctx->device, &scratch);
     if (rc != HT_OK) return rc;
     int bpsm = 0;
-    rc = walk_blocks_per_sm<false>(&bpsm);
+    rc = walk_blocks_per_sm<false, 3>(&bpsm);
     if (rc != HT_OK) return rc;
     if (ctx->tune_walk_bpsm > 0 && ctx->tune_walk_bpsm < bpsm) bpsm = ctx->tune_walk_bpsm;
     long long blocks = (long long)ctx->num_sms * bpsm;
@@ -1512,7 +1526,7 @@ extern "C" HT_API int ht_shell_analyse_static(ht_ctx* ctx, const ht_fields* f,
     a.queue = nullptr; a.dynamic = 0;   // static item-to-warp schedule: no counter to clear
     a.stats = nullptr;
     const size_t smem = walk_smem_bytes();
-    walk_kernel<false><<<(unsigned)blocks, kThreads, smem, (cudaStream_t)stream>>>(a);
+    walk_kernel<false, 3><<<(unsigned)blocks, kThreads, smem, (cudaStream_t)stream>>>(a);
     HT_CUDA_TRY(cudaGetLastError(), "walk_kernel launch (static scratch)");
     ctx->last_kernels = 1;
     return HT_OK;
