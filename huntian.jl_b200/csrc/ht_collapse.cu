@@ -7,7 +7,15 @@
 // One thread integrates one ellipsoid in FP64; the entries are independent (20,000 for the
 // 50 x 20 x 20 table).  The integration is a dependent chain of ~10^3 RK4 steps, each four
 // right-hand sides with two Carlson RD evaluations (square-root chains): latency bound, so
-// the launch uses small CTAs to spread the threads over every SM.  This file is compiled
+// the launch uses small CTAs to spread the threads over every SM, and the chain is kept
+// short: the two RD sets advance in one branch-free round whose stopping test needs no
+// division, what depends on the time alone is evaluated side by side for all times of a
+// step, and a division by a tabulated or shared number is a product with its reciprocal
+// and one correction (quot).  All of it leaves every bit as it was.  The default table:
+// 326 -> 124 ms by RK4 (straight-line roots and reciprocals, which overlap, took it from 220
+// to 138; entries in the order of their lengths from 138 to 124), 6.2 -> 3.5 ms by Tsit5.
+// What is left is the FP64 issue of one or two warps per scheduler: taking the next round's
+// roots before the stopping test changed nothing.  This file is compiled
 // with -fmad=false: no product is fused into an addition, the operations run in the
 // reference's order, and the one logarithm on the path (the oblate shape branch) is a
 // series both sides carry, so the results follow the CPU restatement to the last bit.
@@ -19,15 +27,69 @@
 namespace {
 
 constexpr int kRdMaxIt = 200;   // Carlson RD: rounds before the loop gives up (see below)
-constexpr int kEvolveThreads = 64;
+constexpr int kEvolveThreads = 32;   // one warp: CTAs spread over the SMs' schedulers
 
 struct GrowthDev {
     const double* atab;
     const double* Da;
     const double* f;
+    const double* recip;   // per 4-point window: 1 / (xa[i] - xa[j]), i-major, j != i (nullable)
     int ntab;
     double amin, amax, D_inf, D_a0, HD_inf, HD_a0;
 };
+
+// a / b, correctly rounded, from y = 1 / b correctly rounded: q = a y is within one unit in
+// the last place, the remainder a - b q is exact in one fused operation, and q plus the
+// remainder times y rounds to the quotient (P. Markstein, IBM J. Res. Dev. 34 (1990) 111).
+// For quotients well inside the exponent range; quot_any divides outside it.
+__device__ __forceinline__ double quot(double a, double b, double y) {
+    const double q = a * y;
+    return fma(fma(-b, q, a), y, q);
+}
+
+// 1 / b and sqrt(x), correctly rounded, for arguments in the range kind() admits.  The
+// library's versions branch to a path for extreme arguments after each result, so that
+// several in a row run one after the other; these are straight-line, and the six roots and
+// two reciprocals of an RD round overlap.  Reciprocal: Newton's iteration and a last
+// correction with the exact remainder (Markstein, as above; b's significand all ones, one
+// case in 2^52, can come out one unit off).  Root: Goldschmidt's iteration for g = sqrt(x),
+// h = 1 / (2 sqrt(x)), then g plus the exact remainder x - g g times h (P. Markstein,
+// "Software division and square root using Goldschmidt's algorithms", RNC 6, 2004).
+__device__ __forceinline__ bool kind(double x) { return x > 1e-60 && x < 1e60; }
+__device__ __forceinline__ double recip(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));   // about 20 bits
+    y = fma(y, fma(-b, y, 1.0), y);
+    y = fma(y, fma(-b, y, 1.0), y);
+    return fma(y, fma(-b, y, 1.0), y);
+}
+__device__ __forceinline__ double root(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));   // about 20 bits
+    double g = x * y, h = 0.5 * y;
+    double r = fma(-g, h, 0.5);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    r = fma(-g, h, 0.5);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    return fma(fma(-g, g, x), h, g);
+}
+// Either of the two forms, chosen where a call has looked at its arguments.
+template <bool kKind>
+__device__ __forceinline__ double root_t(double x) { return kKind ? root(x) : sqrt(x); }
+template <bool kKind>
+__device__ __forceinline__ double div_t(double a, double b) {
+    return kKind ? quot(a, b, recip(b)) : a / b;
+}
+
+__device__ __forceinline__ double ratio(double a, double b) {
+    return kind(a) && kind(b) ? quot(a, b, recip(b)) : a / b;
+}
+__device__ __forceinline__ double quot_any(double a, double b, double y) {
+    const double m = fabs(a);
+    return b > 1e-30 && b < 1e30 && m < 1e250 && m > 1e-250 ? quot(a, b, y) : a / b;
+}
 
 struct EllDev {
     double Rvac, Rcurv;   // Omvac / Omnr, Omcurv / Omnr (EllipsoidalCollapse.jl:47-55)
@@ -124,58 +186,101 @@ __device__ double dfnofa(const GrowthDev& g, double ai) {
 // Carlson's RD (EllipsoidalCollapse.jl:62-106), two argument sets side by side: each set
 // runs its own duplication rounds until its own stopping test holds (a finished set stops
 // changing) and then the final formula, so both results are those of two separate calls,
-// while the two square-root / division chains overlap.  Finite positive arguments converge
-// in a few dozen rounds; a set stops after kRdMaxIt rounds at the latest (the reference
-// loops for ever on NaN arguments), as the CPU restatement does.
+// while the two square-root chains overlap: a round computes both sets without a branch and
+// keeps the unfinished ones.  Finite positive arguments converge in a few dozen rounds; a
+// set stops after kRdMaxIt rounds at the latest (the reference loops for ever on NaN
+// arguments), as the CPU restatement does.
 struct RdState {
-    double xt, yt, zt, sum, fac, delx, dely, delz, ave;
+    double xt, yt, zt, sum, fac, ave;
     bool done;
 };
 
 __device__ __forceinline__ void rd_init(RdState& r, double x, double y, double z) {
-    r.xt = x; r.yt = y; r.zt = z; r.sum = 0.0; r.fac = 1.0;
-    r.delx = r.dely = r.delz = r.ave = 0.0;
+    r.xt = x; r.yt = y; r.zt = z; r.sum = 0.0; r.fac = 1.0; r.ave = 0.0;
     r.done = false;
 }
 
-__device__ __forceinline__ void rd_round(RdState& r) {
-    const double ERRTOL = 0.05;
-    const double sqrtx = sqrt(r.xt), sqrty = sqrt(r.yt), sqrtz = sqrt(r.zt);
-    const double alamb = sqrtx * (sqrty + sqrtz) + sqrty * sqrtz;
-    r.sum += r.fac / (sqrtz * (r.zt + alamb));
-    r.fac *= 0.25;
-    r.xt = 0.25 * (r.xt + alamb);
-    r.yt = 0.25 * (r.yt + alamb);
-    r.zt = 0.25 * (r.zt + alamb);
-    r.ave = 0.2 * (r.xt + r.yt + 3.0 * r.zt);
-    r.delx = (r.ave - r.xt) / r.ave;
-    r.dely = (r.ave - r.yt) / r.ave;
-    r.delz = (r.ave - r.zt) / r.ave;
-    r.done = fmax(fmax(fabs(r.delx), fabs(r.dely)), fabs(r.delz)) <= ERRTOL;
+constexpr double kRdErrTol = 0.05;
+
+// The stopping test: max |ave - v| / ave, each quotient rounded, within kRdErrTol.  Beyond
+// 1e-14 of the line a product decides it (rounding moves either side by a few 1e-16); on
+// the line, and where a value is not finite, rd_stop takes the quotients.
+struct RdTest { bool yes, open; };
+__device__ __forceinline__ RdTest rd_test(const RdState& r) {
+    const double e = fmax(fmax(fabs(r.ave - r.xt), fabs(r.ave - r.yt)), fabs(r.ave - r.zt));
+    const double line = kRdErrTol * fabs(r.ave);
+    const bool yes = e < line * (1.0 - 1e-14) && line < 1e300;
+    const bool no = e > line * (1.0 + 1e-14) && e < 1e300;
+    return RdTest{yes || r.done, !yes && !no && !r.done};
+}
+__device__ __forceinline__ bool rd_stop(const RdState& r) {
+    const double ave = r.ave;
+    return fmax(fmax(fabs((ave - r.xt) / ave), fabs((ave - r.yt) / ave)),
+                fabs((ave - r.zt) / ave)) <= kRdErrTol;
 }
 
+template <bool kKind>
+__device__ __forceinline__ void rd_round(RdState& r) {
+    const double sqrtx = root_t<kKind>(r.xt), sqrty = root_t<kKind>(r.yt),
+                 sqrtz = root_t<kKind>(r.zt);
+    const double alamb = sqrtx * (sqrty + sqrtz) + sqrty * sqrtz;
+    // (r.fac is a power of two: r.fac times the rounded reciprocal is the rounded quotient)
+    const double den = sqrtz * (r.zt + alamb);
+    const double sum = r.sum + (kKind ? r.fac * recip(den) : r.fac / den);
+    const double xt = 0.25 * (r.xt + alamb), yt = 0.25 * (r.yt + alamb),
+                 zt = 0.25 * (r.zt + alamb);
+    const double ave = 0.2 * (xt + yt + 3.0 * zt);
+    const bool keep = r.done;
+    r.sum = keep ? r.sum : sum;
+    r.fac = keep ? r.fac : r.fac * 0.25;
+    r.xt = keep ? r.xt : xt;
+    r.yt = keep ? r.yt : yt;
+    r.zt = keep ? r.zt : zt;
+    r.ave = keep ? r.ave : ave;
+}
+
+template <bool kKind>
 __device__ __forceinline__ double rd_final(const RdState& r) {
     const double C1 = 3.0 / 14.0, C2 = 1.0 / 6.0, C3 = 9.0 / 22.0, C4 = 3.0 / 26.0,
                  C5 = 0.25 * C3, C6 = 1.5 * C4;
-    const double delx = r.delx, dely = r.dely, delz = r.delz, ave = r.ave;
+    const double ave = r.ave, delx = div_t<kKind>(ave - r.xt, ave),
+                 dely = div_t<kKind>(ave - r.yt, ave), delz = div_t<kKind>(ave - r.zt, ave);
     const double ea = delx * dely, eb = delz * delz, ec = ea - eb, ed = ea - 6.0 * eb,
                  ee = ed + ec + ec;
-    return 3.0 * r.sum + r.fac * (1.0 + ed * (-C1 + C5 * ed - C6 * delz * ee) +
-                                  delz * (C2 * ee + delz * (-C3 * ec + delz * C4 * ea))) /
-                             (ave * sqrt(ave));
+    return 3.0 * r.sum +
+           div_t<kKind>(r.fac * (1.0 + ed * (-C1 + C5 * ed - C6 * delz * ee) +
+                                 delz * (C2 * ee + delz * (-C3 * ec + delz * C4 * ea))),
+                        ave * root_t<kKind>(ave));
 }
 
-__device__ void elliptic_rd2(double x1, double y1, double z1, double x2, double y2, double z2,
-                             double* r1, double* r2) {
+template <bool kKind>
+__device__ __forceinline__ void rd_pair(RdState& a, RdState& b, double* r1, double* r2) {
+    for (int it = 0; it < kRdMaxIt && !(a.done && b.done); ++it) {
+        rd_round<kKind>(a);
+        rd_round<kKind>(b);
+        const RdTest ta = rd_test(a), tb = rd_test(b);
+        a.done = ta.yes;
+        b.done = tb.yes;
+        if (ta.open || tb.open) {
+            if (ta.open) a.done = rd_stop(a);
+            if (tb.open) b.done = rd_stop(b);
+        }
+    }
+    *r1 = rd_final<kKind>(a);
+    *r2 = rd_final<kKind>(b);
+}
+
+__device__ __forceinline__ void elliptic_rd2(double x1, double y1, double z1, double x2,
+                                             double y2, double z2, double* r1, double* r2) {
     RdState a, b;
     rd_init(a, x1, y1, z1);
     rd_init(b, x2, y2, z2);
-    for (int it = 0; it < kRdMaxIt && !(a.done && b.done); ++it) {
-        if (!a.done) rd_round(a);
-        if (!b.done) rd_round(b);
-    }
-    *r1 = rd_final(a);
-    *r2 = rd_final(b);
+    // a round keeps the arguments between a quarter of the least and the largest of them
+    auto fits = [](double x) { return x > 1e-12 && x < 1e12; };
+    if (fits(x1) && fits(y1) && fits(z1) && fits(x2) && fits(y2) && fits(z2))
+        rd_pair<true>(a, b, r1, r2);
+    else
+        rd_pair<false>(a, b, r1, r2);
 }
 
 // Natural log of a finite x > 0 (and log2 x through log2x when non-null): x = m 2^e with m
@@ -189,6 +294,7 @@ __device__ double log_series(double x, double* log2x) {
     if (m < 0.7071067811865476) { m *= 2.0; ex -= 1; }
     const double s = (m - 1.0) / (m + 1.0), s2 = s * s;
     double t = 1.0 / 23.0;
+#pragma unroll
     for (int k = 21; k >= 1; k -= 2) t = 1.0 / (double)k + s2 * t;
     const double lnm = 2.0 * s * t;
     if (log2x) *log2x = (double)ex + lnm * 1.4426950408889634;
@@ -198,7 +304,9 @@ __device__ double log_series(double x, double* log2x) {
 // Shape integrals (EllipsoidalCollapse.jl:108-146, iwant_rd = 1).
 __device__ void get_b_2(double a1, double a2, double a3, double* b) {
     const double third = 1.0 / 3.0;
-    const double r_2 = a2 / a1, r_3 = a3 / a1;
+    const bool fine = kind(a1) && kind(a2) && kind(a3);
+    const double ia1 = recip(a1);
+    const double r_2 = fine ? quot(a2, a1, ia1) : a2 / a1, r_3 = fine ? quot(a3, a1, ia1) : a3 / a1;
     if (r_3 >= r_2) {
         if (r_3 >= 0.999) {
             b[0] = b[1] = b[2] = third;
@@ -234,7 +342,6 @@ __device__ void get_b_2(double a1, double a2, double a3, double* b) {
 // DerivState (EllipsoidalCollapse.jl:174-191).
 struct DState {
     int lvirv[3];
-    int hint;             // growth-table index of the last lookup
     double a_3eq, a_2eq, a_1eq, a_3eq2, a_3eq1, Ha;
     double aLam[3], Frho_3;
 };
@@ -243,16 +350,101 @@ __device__ double ha_b_nr(double a_b, const EllDev& e) {
     return sqrt((1.0 + e.Rvac * (a_b * a_b * a_b) + e.Rcurv * a_b) / a_b);
 }
 
+// What the right-hand sides need of the time t = a alone: the Hubble rate, the background
+// and external-tide coefficients.
+struct TimeTerms {
+    double a_b, a_b3, ia_b3, Ha, Ha_inv, d0, d1_ext;
+};
+
+// The terms of N times at once; *hint: the growth-table index of the last lookup.  The N
+// chains (a division, a square root, a division, and the three divisions in a row of each
+// Lagrange weight) run side by side.
+template <int N>
+__device__ __forceinline__ void time_terms(const EllDev& e, const GrowthDev& g,
+                                           const double (&t)[N], TimeTerms (&o)[N], int* hint) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        TimeTerms& q = o[i];
+        q.a_b = t[i];
+        q.a_b3 = t[i] * t[i] * t[i];
+        // ha_b_nr and two reciprocals
+        const double num = 1.0 + e.Rvac * q.a_b3 + e.Rcurv * t[i];
+        const double arg = quot(num, t[i], recip(t[i]));
+        q.Ha = root(arg);
+        q.Ha_inv = recip(q.Ha);
+        q.ia_b3 = recip(q.a_b3);
+        if (!(t[i] > 1e-15 && t[i] < 1e15 && kind(num) && kind(arg))) {
+            q.Ha = ha_b_nr(t[i], e);
+            q.Ha_inv = 1.0 / q.Ha;
+            q.ia_b3 = 1.0 / q.a_b3;
+        }
+        q.d0 = e.fs == 0 ? -e.Rvac * q.Ha_inv : (0.5 * q.ia_b3 - e.Rvac) * q.Ha_inv;
+        q.d1_ext = e.fs == 3 ? 1.5 * 2.5 / q.a_b3 * q.Ha_inv : 0.0;
+    }
+    if (e.fs != 4 && e.fs != 5 && e.fs != 6) return;
+    double dlin[N];
+    int k0[N];
+    bool four = g.recip != nullptr;   // every time inside the table, with a 4-point window
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const bool in = t[i] > g.amin && t[i] < g.amax;
+        const int kk = in ? (*hint = hunt_from(g.atab, g.ntab, t[i], *hint)) : 0;
+        k0[i] = (kk - 2 > 1 ? kk - 2 : 1) - 1;
+        four = four && in && kk >= 2 && kk < g.ntab;
+    }
+    if (four) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const double *xa = g.atab + k0[i], *y = g.recip + 12 * k0[i], *v = g.Da + k0[i];
+            double x[4], d[4], w[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                x[j] = __ldg(xa + j);
+                d[j] = t[i] - x[j];
+            }
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {   // the factors in the order of growth_weights
+                const int j0 = p == 0 ? 1 : 0, j1 = p <= 1 ? 2 : 1, j2 = p <= 2 ? 3 : 2;
+                double q = quot(d[j0], x[p] - x[j0], __ldg(y + 3 * p));
+                q = quot(q * d[j1], x[p] - x[j1], __ldg(y + 3 * p + 1));
+                w[p] = quot(q * d[j2], x[p] - x[j2], __ldg(y + 3 * p + 2));
+            }
+            dlin[i] = (w[0] * __ldg(v) + w[1] * __ldg(v + 1) + w[2] * __ldg(v + 2) +
+                       w[3] * __ldg(v + 3)) * t[i];
+        }
+    } else {
+        for (int i = 0; i < N; ++i) {
+            double hd;
+            dlinear_ab(g, t[i], &dlin[i], &hd, hint);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+        o[i].d1_ext = quot_any(1.5, o[i].a_b3, o[i].ia_b3) * o[i].Ha_inv * dlin[i];
+}
+
+__device__ __forceinline__ TimeTerms time_terms1(const EllDev& e, const GrowthDev& g, double t,
+                                                 int* hint) {
+    const double ts[1] = {t};
+    TimeTerms o[1];
+    time_terms<1>(e, g, ts, o, hint);
+    return o[0];
+}
+
+// 1.5 x / a^3 Ha_inv, the coefficient of the ellipsoid's own field.
+__device__ __forceinline__ double interior_coef(const TimeTerms& q, double x) {
+    return quot_any(1.5 * x, q.a_b3, q.ia_b3) * q.Ha_inv;
+}
+
 // get_derivs! (EllipsoidalCollapse.jl:200-290): dy at (t, y); freezes the virialised axes
 // in y and advances the flags (also from the intermediate RK4 stages, as the Fortran does).
-__device__ void get_derivs(const EllDev& e, const GrowthDev& g, double t, double* y,
-                           double* dy, DState& ds) {
+__device__ void get_derivs(const EllDev& e, const TimeTerms& q, double* y, double* dy,
+                           DState& ds) {
 #pragma unroll
     for (int i = 0; i < 6; ++i) dy[i] = 0.0;
-    const double a_b = t, a_b3 = a_b * a_b * a_b;
-    const double Ha = ha_b_nr(a_b, e);
-    ds.Ha = Ha;
-    const double Ha_inv = 1.0 / Ha;
+    const double a_b = q.a_b, a_b3 = q.a_b3;
+    ds.Ha = q.Ha;
+    const double Ha_inv = q.Ha_inv;
     if (ds.lvirv[2] == 0 && y[2] <= e.fcoll[2] * a_b) {
         ds.lvirv[2] = 1;
         ds.a_3eq = e.fcoll[2] * a_b;
@@ -276,22 +468,9 @@ __device__ void get_derivs(const EllDev& e, const GrowthDev& g, double t, double
     if (ds.lvirv[0] == 1) { y[0] = ds.a_1eq; y[3] = 0.0; dy[0] = 0.0; dy[3] = 0.0; }
 
     const double a1 = y[0], a2 = y[1], a3 = y[2];
-    const double delta1_e = a_b3 / (a1 * a2 * a3);
-    double d0, d1_int, d1_ext = 0.0;
-    if (e.fs == 0) {
-        d0 = -e.Rvac * Ha_inv;
-        d1_int = 1.5 * delta1_e / a_b3 * Ha_inv;
-    } else {
-        d0 = (0.5 / a_b3 - e.Rvac) * Ha_inv;
-        d1_int = 1.5 * (delta1_e - 1.0) / a_b3 * Ha_inv;
-        if (e.fs == 4 || e.fs == 5 || e.fs == 6) {
-            double dlin, hd;
-            dlinear_ab(g, a_b, &dlin, &hd, &ds.hint);
-            d1_ext = 1.5 / a_b3 * Ha_inv * dlin;
-        } else if (e.fs == 3) {
-            d1_ext = 1.5 * 2.5 / a_b3 * Ha_inv;
-        }
-    }
+    const double delta1_e = ratio(a_b3, a1 * a2 * a3);
+    const double d0 = q.d0, d1_ext = q.d1_ext;
+    const double d1_int = interior_coef(q, e.fs == 0 ? delta1_e : delta1_e - 1.0);
     double b[3] = {0.0, 0.0, 0.0};
     if (e.fs != 5 && e.fs != 6) get_b_2(a1, a2, a3, b);
     const double third = 1.0 / 3.0;
@@ -311,23 +490,24 @@ __device__ void get_derivs(const EllDev& e, const GrowthDev& g, double t, double
 }
 
 // One step of rk4_homel! (EllipsoidalCollapse.jl:149-172); dy holds the derivatives at
-// (t, y).
-__device__ void rk4_step(const EllDev& e, const GrowthDev& g, const double* y,
-                         const double* dy, double t, double h, double* yout, DState& ds) {
+// (t, y), mid and end the terms of t + h / 2 and t + h.
+__device__ void rk4_step(const EllDev& e, const TimeTerms& mid, const TimeTerms& end,
+                         const double* y, const double* dy, double h, double* yout,
+                         DState& ds) {
     double yt[6], dyt[6], dym[6];
-    const double hh = h * 0.5, h6 = h / 6.0, xh = t + hh;
+    const double hh = h * 0.5, h6 = h / 6.0;
 #pragma unroll
     for (int i = 0; i < 6; ++i) yt[i] = y[i] + hh * dy[i];
-    get_derivs(e, g, xh, yt, dyt, ds);
+    get_derivs(e, mid, yt, dyt, ds);
 #pragma unroll
     for (int i = 0; i < 6; ++i) yt[i] = y[i] + hh * dyt[i];
-    get_derivs(e, g, xh, yt, dym, ds);
+    get_derivs(e, mid, yt, dym, ds);
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
         yt[i] = y[i] + h * dym[i];
         dym[i] = dyt[i] + dym[i];
     }
-    get_derivs(e, g, t + h, yt, dyt, ds);
+    get_derivs(e, end, yt, dyt, ds);
 #pragma unroll
     for (int i = 0; i < 6; ++i) yout[i] = y[i] + h6 * (dy[i] + dyt[i] + 2.0 * dym[i]);
 }
@@ -346,7 +526,7 @@ __global__ void __launch_bounds__(kEvolveThreads) evolve_kernel(
     const double Frho = Frho_in[q], e_v = ev_in[q], p_v = pv_in[q];
     DState ds;
     ds.lvirv[0] = ds.lvirv[1] = ds.lvirv[2] = 0;
-    ds.hint = 0;
+    int hint = 0;
     ds.a_3eq = ds.a_2eq = ds.a_1eq = ds.a_3eq2 = ds.a_3eq1 = 0.0;
     ds.aLam[2] = Frho / 3.0 * (1.0 + 3.0 * e_v + p_v);
     ds.aLam[1] = Frho / 3.0 * (1.0 - 2.0 * p_v);
@@ -368,13 +548,19 @@ __global__ void __launch_bounds__(kEvolveThreads) evolve_kernel(
 #pragma unroll
     for (int i = 0; i < 6; ++i) { zdynv[i] = -1.0; ldynv[i] = 0; }
     int istep = 0;
+    TimeTerms now = time_terms1(e, g, t, &hint);
     // bounded: every round advances istep, and the loop ends at nstepmax
     for (;;) {
         ++istep;
         const double a_3 = y[2];
-        const double dtstep = e.tfac * a_3 * sqrt(a_3) * ds.Ha;
-        get_derivs(e, g, t, y, dy, ds);
-        rk4_step(e, g, y, dy, t, dtstep, yout, ds);
+        const double dtstep = e.tfac * a_3 * (kind(a_3) ? root(a_3) : sqrt(a_3)) * ds.Ha;
+        // the terms of the step's middle and end; the end is the next step's beginning
+        const double ts[2] = {t + dtstep * 0.5, t + dtstep};
+        TimeTerms tt[2];
+        time_terms<2>(e, g, ts, tt, &hint);
+        get_derivs(e, now, y, dy, ds);
+        rk4_step(e, tt[0], tt[1], y, dy, dtstep, yout, ds);
+        now = tt[1];
 #pragma unroll
         for (int i = 0; i < 6; ++i) y[i] = yout[i];
         t += dtstep;
@@ -431,25 +617,23 @@ __device__ double pow_pos(double x, double y) {
     const double nn = floor(v + 0.5);
     const double f = (v - nn) * 0.6931471805599453;
     double p = 1.0;
-    for (int k = 16; k >= 1; --k) p = 1.0 + f * p / (double)k;
+#pragma unroll
+    for (int k = 16; k >= 1; --k) p = 1.0 + quot(f * p, (double)k, 1.0 / (double)k);
     return ldexp(p, (int)nn);
 }
 
-// VirState (EllipsoidalCollapse.jl:327-333), with the growth-table lookup hint.
+// VirState (EllipsoidalCollapse.jl:327-333).
 struct VirDev {
     int lvirv[3];
-    int hint;
     double a_eq[3], zdynv[3];
 };
 
 // _diffeq_rhs! (EllipsoidalCollapse.jl:344-438): du at (t, u); freezes the virialised axes
 // in u and advances the flags at every evaluation (accepted step or not), recording 1/a at
 // the evaluation that sets each.  aLam[3] = Frho / 3; iforce_strat 2 keeps the velocities.
-__device__ void diffeq_rhs(const EllDev& e, const GrowthDev& g, const double* aLam, double t,
-                           double* u, double* du, VirDev& v) {
-    const double a_b = t, a_b3 = a_b * a_b * a_b;
-    const double Ha = ha_b_nr(a_b, e);
-    const double Ha_inv = 1.0 / Ha;
+__device__ void diffeq_rhs(const EllDev& e, const TimeTerms& q, const double* aLam, double* u,
+                           double* du, VirDev& v) {
+    const double a_b = q.a_b, a_b3 = q.a_b3, Ha_inv = q.Ha_inv;
     if (v.lvirv[2] == 0 && u[2] <= e.fcoll[2] * a_b) {
         v.lvirv[2] = 1;
         v.a_eq[2] = e.fcoll[2] * a_b;
@@ -475,23 +659,10 @@ __device__ void diffeq_rhs(const EllDev& e, const GrowthDev& g, const double* aL
         if (v.lvirv[ax] == 1) { u[ax] = v.a_eq[ax]; u[ax + 3] = 0.0; }
 
     const double a1 = u[0], a2 = u[1], a3 = u[2];
-    const double delta1_e = a_b3 / (a1 * a2 * a3);
+    const double delta1_e = ratio(a_b3, a1 * a2 * a3);
     const double Frho_3 = aLam[3];
-    double d0, d1_int, d1_ext = 0.0;
-    if (e.fs == 0) {
-        d0 = -e.Rvac * Ha_inv;
-        d1_int = 1.5 * delta1_e / a_b3 * Ha_inv;
-    } else {
-        d0 = (0.5 / a_b3 - e.Rvac) * Ha_inv;
-        d1_int = 1.5 * (delta1_e - 1.0) / a_b3 * Ha_inv;
-        if (e.fs == 4 || e.fs == 5 || e.fs == 6) {
-            double dlin, hd;
-            dlinear_ab(g, a_b, &dlin, &hd, &v.hint);
-            d1_ext = 1.5 / a_b3 * Ha_inv * dlin;
-        } else if (e.fs == 3) {
-            d1_ext = 1.5 * 2.5 / a_b3 * Ha_inv;
-        }
-    }
+    const double d0 = q.d0, d1_ext = q.d1_ext;
+    const double d1_int = interior_coef(q, e.fs == 0 ? delta1_e : delta1_e - 1.0);
     double b[3] = {0.0, 0.0, 0.0};
     if (e.fs != 5 && e.fs != 6) get_b_2(a1, a2, a3, b);
     const double third = 1.0 / 3.0;
@@ -555,13 +726,13 @@ __global__ void __launch_bounds__(kEvolveThreads) evolve_tsit5_kernel(
     aLam[0] = Frho / 3.0 * (1.0 - 3.0 * e_v + p_v);
     aLam[3] = Frho / 3.0;
     VirDev v;
-    v.hint = 0;
+    int hint = 0;
 #pragma unroll
     for (int i = 0; i < 3; ++i) { v.lvirv[i] = 0; v.a_eq[i] = 0.0; v.zdynv[i] = -1.0; }
     const double zinit = e.zinit_fac * Frho;
     const double a_b = 1.0 / zinit;
     double dlin, HD_Ha;
-    dlinear_ab(g, a_b, &dlin, &HD_Ha, &v.hint);
+    dlinear_ab(g, a_b, &dlin, &HD_Ha, &hint);
     const double Ha = ha_b_nr(a_b, e);
     double u[6];
 #pragma unroll
@@ -571,7 +742,8 @@ __global__ void __launch_bounds__(kEvolveThreads) evolve_tsit5_kernel(
     double t = a_b;
 
     double k[7][6], tmp[6], sc[6], u1[6];
-    diffeq_rhs(e, g, aLam, t, u, k[0], v);
+    const TimeTerms first = time_terms1(e, g, t, &hint);
+    diffeq_rhs(e, first, aLam, u, k[0], v);
 #pragma unroll
     for (int i = 0; i < 6; ++i) sc[i] = abstol + fabs(u[i]) * reltol;
 #pragma unroll
@@ -584,7 +756,7 @@ __global__ void __launch_bounds__(kEvolveThreads) evolve_tsit5_kernel(
     if (dt0 > tend - t) dt0 = tend - t;
 #pragma unroll
     for (int i = 0; i < 6; ++i) u1[i] = u[i] + dt0 * k[0][i];
-    diffeq_rhs(e, g, aLam, t + dt0, u1, k[1], v);
+    diffeq_rhs(e, time_terms1(e, g, t + dt0, &hint), aLam, u1, k[1], v);
 #pragma unroll
     for (int i = 0; i < 6; ++i) tmp[i] = (k[1][i] - k[0][i]) / sc[i];
     const double d2 = rms6(tmp) / dt0;
@@ -593,7 +765,7 @@ __global__ void __launch_bounds__(kEvolveThreads) evolve_tsit5_kernel(
                                      : pow_pos(0.01 / dmax, 0.2);
     double dt = 100.0 * dt0 < dt1 ? 100.0 * dt0 : dt1;
     if (dt > tend - t) dt = tend - t;
-    diffeq_rhs(e, g, aLam, t, u, k[0], v);   // the first FSAL stage
+    diffeq_rhs(e, first, aLam, u, k[0], v);   // the first FSAL stage
 
     double qold = 1e-4;
     int iter = 0;
@@ -602,6 +774,12 @@ __global__ void __launch_bounds__(kEvolveThreads) evolve_tsit5_kernel(
         ++iter;
         if (dt > tend - t) dt = tend - t;
         if (!(dt > 1e-14 * t)) break;   // step size underflow: give up
+        // stages 5 and 6 share their time
+        double ts[5];
+        TimeTerms tt[5];
+#pragma unroll
+        for (int st = 1; st < 6; ++st) ts[st - 1] = t + kTsC[st] * dt;
+        time_terms<5>(e, g, ts, tt, &hint);
         for (int st = 1; st < 7; ++st) {
 #pragma unroll
             for (int i = 0; i < 6; ++i) {
@@ -609,7 +787,7 @@ __global__ void __launch_bounds__(kEvolveThreads) evolve_tsit5_kernel(
                 for (int j = 0; j < st; ++j) acc += kTsA[st][j] * k[j][i];
                 tmp[i] = u[i] + dt * acc;
             }
-            diffeq_rhs(e, g, aLam, t + kTsC[st] * dt, tmp, k[st], v);
+            diffeq_rhs(e, tt[st < 6 ? st - 1 : 4], aLam, tmp, k[st], v);
         }
         // tmp is the step's end, frozen by the last evaluation
         double r[6];
@@ -723,17 +901,40 @@ extern "C" HT_API int ht_evolve_ellipses(int device, const ht_ellipsoid* ep,
         return ht_fail(HT_ERR_INVALID, "ht_evolve_ellipses: NULL input or output array");
     HT_CUDA_TRY(cudaSetDevice(device), "ht_evolve_ellipses: cudaSetDevice");
     cudaStream_t st = (cudaStream_t)stream;
+    // the growth table and the reciprocals of its 4-point windows, in one upload
     const int nt = growth->ntab;
-    const size_t tb = (size_t)nt * sizeof(double);
+    std::vector<double> h(growth->atab, growth->atab + nt);
+    h.insert(h.end(), growth->D_atab, growth->D_atab + nt);
+    h.insert(h.end(), growth->dlnD_dlnatab, growth->dlnD_dlnatab + nt);
+    // (while a graph is captured the copies must come from the caller's own arrays, which
+    // outlive this call: no reciprocals then)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    HT_CUDA_TRY(cudaStreamIsCapturing(st, &cap), "ht_evolve_ellipses: stream state");
+    const bool capturing = cap != cudaStreamCaptureStatusNone;
+    bool tame = !capturing;   // and spacings for which quot holds
+    for (int k = 0; tame && k + 3 < nt; ++k)
+        for (int i = 0; i < 4; ++i)
+            for (int j = 0; j < 4; ++j) {
+                if (j == i) continue;
+                const double d = growth->atab[k + i] - growth->atab[k + j];
+                tame = tame && std::fabs(d) > 1e-12 && std::fabs(d) < 1e12;
+                h.push_back(1.0 / d);
+            }
     double* buf = nullptr;
-    HT_CUDA_TRY(cudaMallocAsync((void**)&buf, 3 * tb, st), "ht_evolve_ellipses: growth table");
-    cudaError_t e = cudaMemcpyAsync(buf, growth->atab, tb, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(buf + nt, growth->D_atab, tb, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(buf + 2 * nt, growth->dlnD_dlnatab, tb, cudaMemcpyHostToDevice, st);
+    HT_CUDA_TRY(cudaMallocAsync((void**)&buf, h.size() * sizeof(double), st),
+                "ht_evolve_ellipses: growth table");
+    cudaError_t e = cudaSuccess;
+    if (capturing) {
+        const double* part[3] = {growth->atab, growth->D_atab, growth->dlnD_dlnatab};
+        for (int i = 0; i < 3 && e == cudaSuccess; ++i)
+            e = cudaMemcpyAsync(buf + (size_t)i * nt, part[i], (size_t)nt * sizeof(double),
+                                cudaMemcpyHostToDevice, st);
+    } else {
+        e = cudaMemcpyAsync(buf, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, st);
+    }
     if (e == cudaSuccess) {
-        GrowthDev g{buf, buf + nt, buf + 2 * nt, nt, growth->amintab, growth->amaxtab,
+        GrowthDev g{buf, buf + nt, buf + 2 * nt, tame ? buf + 3 * nt : nullptr, nt,
+                    growth->amintab, growth->amaxtab,
                     growth->D_ainfty, growth->D_a0, growth->HD_Hainfty, growth->HD_Ha0};
         const long long blocks = (n + kEvolveThreads - 1) / kEvolveThreads;
         if (ep->solver == HT_SOLVER_TSIT5)
@@ -768,11 +969,16 @@ extern "C" HT_API int ht_collapse_table(int device, const ht_ellipsoid* ep,
     // the grid of CollapseTable.jl:29-50 on the host (10^x with the host's pow, as the
     // CPU restatement and Julia's 10.0^logF)
     const double dX = (X2 - X1) / (nx - 1), dY = (Y2 - Y1) / (ny - 1), dZ = (Z2 - Z1) / (nz - 1);
-    std::vector<double> h(3 * (size_t)n);
+    std::vector<double> h(3 * (size_t)n), Frho(nx);
+    for (int i = 0; i < nx; ++i) Frho[i] = std::pow(10.0, X1 + i * dX);
+    // e_v slowest and from its largest value down: the RK4's steps go with e_v first (650 to
+    // 10,000 over the default table), so that a warp's entries take about as long, and the
+    // long warps start first, each on a scheduler of its own
     for (long long q = 0; q < n; ++q) {
-        const int i = (int)(q % nx), j = (int)((q / nx) % ny), k = (int)(q / ((long long)nx * ny));
-        const double x = X1 + i * dX, y = Y1 + j * dY, z = Z1 + k * dZ;
-        h[q] = std::pow(10.0, x);
+        const int i = (int)(q % nx), k = (int)((q / nx) % nz),
+                  j = ny - 1 - (int)(q / ((long long)nx * nz));
+        const double y = Y1 + j * dY, z = Z1 + k * dZ;
+        h[q] = Frho[i];
         h[n + q] = y;
         h[2 * n + q] = z * y;
     }
@@ -792,6 +998,9 @@ extern "C" HT_API int ht_collapse_table(int device, const ht_ellipsoid* ep,
     }
     cudaFree(d);
     if (rc != HT_OK) return rc;
-    for (long long q = 0; q < n; ++q) table[q] = (float)h[q];
+    for (long long q = 0; q < n; ++q) {
+        const long long i = q % nx, k = (q / nx) % nz, j = ny - 1 - q / ((long long)nx * nz);
+        table[i + nx * (j + ny * k)] = (float)h[q];
+    }
     return HT_OK;
 }

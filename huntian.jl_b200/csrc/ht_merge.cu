@@ -122,6 +122,7 @@ __global__ void iota_kernel(int32_t* __restrict__ v, long long n) {
 }
 
 enum : uint8_t { kUndecided = 0, kAlive = 1, kDead = 2 };
+constexpr int kBigThreads = 64;   // a big halo's CTA
 
 // The halos in cell order: position and radius, place in the sweep order (rank), and the
 // cells' ranges.  A row of cells along x is one contiguous range, so a search reads
@@ -155,13 +156,16 @@ __device__ __forceinline__ Box box_of(const Grid& g, const float4& v, double rea
                cell1(v.z - R, g.z0, g.cs, g.nc), cell1(v.z + R, g.z0, g.cs, g.nc)};
 }
 
-// Calls f(p) for every halo p in the box's cells: one thread, or (kCta) the CTA's warps
-// over the rows and their lanes along a row.
+// Calls f(p) for every halo p in the box's cells: one thread, or (kCta) a CTA, eight lanes
+// along each row: a big halo just over the line has some ten rows of about five halos, one
+// or two passes for a CTA of 64 threads (with a warp along each row most of its lanes had
+// nothing to read: 866 us of rounds, against 586 with eight lanes in CTAs of 128 threads and
+// 455 with 64; 32 threads or a lower line for `big` gave 780 to 840).
 template <bool kCta, class F>
 __device__ __forceinline__ void for_neighbours(const Nbr& nb, const Box& b, F&& f) {
     const int nc = nb.g.nc, ny = b.y1 - b.y0 + 1, rows = ny * (b.z1 - b.z0 + 1);
-    const int r0 = kCta ? threadIdx.x >> 5 : 0, dr = kCta ? blockDim.x >> 5 : 1;
-    const int l0 = kCta ? threadIdx.x & 31 : 0, dl = kCta ? 32 : 1;
+    const int r0 = kCta ? threadIdx.x >> 3 : 0, dr = kCta ? blockDim.x >> 3 : 1;
+    const int l0 = kCta ? threadIdx.x & 7 : 0, dl = kCta ? 8 : 1;
     for (int r = r0; r < rows; r += dr) {
         const long long row = ((long long)(b.z0 + r / ny) * nc + b.y0 + r % ny) * nc;
         const int e = __ldg(nb.cstart + row + b.x1 + 1);
@@ -191,10 +195,10 @@ __global__ void cell_order_kernel(const int32_t* __restrict__ list, long long n,
 //
 // Bound by the latency of the scattered reads.  With a thread per halo in rank order, the
 // halos reached through a list of ranks, and every cell within ceil(r / cell) of the
-// centre, the rounds of a 2.0 M catalogue took 13.2 ms; they take 1.7 ms (half of it the
+// centre, the rounds of a 2.0 M catalogue took 13.2 ms; they take 1.1 ms (40 % of it the
 // 36,000 big halos) with rows of cells as ranges and the box of the radius itself.
 template <bool kCta>
-__global__ void __launch_bounds__(kCta ? 128 : 256) push_kernel(
+__global__ void __launch_bounds__(kCta ? kBigThreads : 256) push_kernel(
     Nbr nb, long long n, const uint8_t* __restrict__ status,
     const int32_t* __restrict__ alive_round, int round,
     const unsigned long long* __restrict__ left, uint8_t* __restrict__ blocked,
@@ -262,7 +266,7 @@ __device__ __forceinline__ void sphere_overlap(double d, double r1, double r2, d
 }
 
 template <bool kCta>
-__global__ void __launch_bounds__(kCta ? 128 : 256) overlap_kernel(
+__global__ void __launch_bounds__(kCta ? kBigThreads : 256) overlap_kernel(
     Nbr nb, long long n, const uint8_t* __restrict__ status, bool fortran_ties,
     double* __restrict__ dV) {
     auto visit = [&](int s) {
@@ -578,7 +582,7 @@ extern "C" HT_API int ht_merge_halos(ht_ctx* ctx, const float* d_records, int64_
     HT_CUDA_TRY(cudaMemsetAsync(nbig, 0, sizeof(int32_t), st), "big count reset");
     cell_order_kernel<<<blocks, 256, 0, st>>>(l1, n, xyzr, big, cxyzr, open_rank, at, nbig);
     HT_CUDA_TRY(cudaGetLastError(), "cell_order_kernel launch");
-    const unsigned big_ctas = (unsigned)std::min<long long>(n, 16LL * ctx->num_sms);
+    const unsigned big_ctas = (unsigned)std::min<long long>(n, 32LL * ctx->num_sms);
     // ---- exclusion rounds ----
     HT_CUDA_TRY(cudaMemsetAsync(status, kUndecided, 3 * (size_t)n, st), "status and marks reset");
     HT_CUDA_TRY(cudaMemsetAsync(alive_round, 0xff, n * sizeof(int32_t), st), "rounds reset");
@@ -592,7 +596,7 @@ extern "C" HT_API int ht_merge_halos(ht_ctx* ctx, const float* d_records, int64_
                     "counter reset");
         for (int k = 0; k < kBatch; ++k, ++rounds) {
             const unsigned long long* before = k ? now + k - 1 : last;
-            push_kernel<true><<<big_ctas, 128, 0, st>>>(nb, n, status, alive_round, rounds, before,
+            push_kernel<true><<<big_ctas, kBigThreads, 0, st>>>(nb, n, status, alive_round, rounds, before,
                                                         blocked, killed);
             push_kernel<false><<<blocks, 256, 0, st>>>(nb, n, status, alive_round, rounds, before,
                                                        blocked, killed);
@@ -614,7 +618,7 @@ extern "C" HT_API int ht_merge_halos(ht_ctx* ctx, const float* d_records, int64_
     const bool reduce = volume_reduction != 0;
     if (reduce) {
         HT_CUDA_TRY(cudaMemsetAsync(dV, 0, n * sizeof(double), st), "dV reset");
-        overlap_kernel<true><<<big_ctas, 128, 0, st>>>(nb, n, status, fortran_ties != 0, dV);
+        overlap_kernel<true><<<big_ctas, kBigThreads, 0, st>>>(nb, n, status, fortran_ties != 0, dV);
         overlap_kernel<false><<<blocks, 256, 0, st>>>(nb, n, status, fortran_ties != 0, dV);
         HT_CUDA_TRY(cudaGetLastError(), "overlap_kernel launch");
     }

@@ -148,3 +148,25 @@ def test_tsit5_table_and_events_match_oracle(ht, planck):
         _compare(D, want[:, 1], step_rel=0.2)
         assert np.mean(st == want[:, 3]) >= 0.99
     assert col.evolve_ellipse_full(0.5, 0.0, 0.0, ep) == (-1.0, -1.0, -1.0)
+
+
+@pytest.mark.parametrize("solver", ["rk4", "diffeq"])
+@pytest.mark.parametrize("shape", [(2, 2, 2), (33, 2, 3), (5, 31, 2)])
+def test_table_order_and_edges(ht, oracle, solver, shape):
+    """Tables whose entries do not fill the last warp, at the extremes of the axes: shapes near
+    the spherical limit (e_v = 0), oblate and prolate ones (p_v / e_v = -1, 1) and radii past
+    the division-free form of the shape integrals' test.  Every entry equals the scalar call."""
+    col = ht.collapse
+    ep = col.EllipsoidParams(ht.catalog.CosmologyParams(Om=0.3, OL=0.7), solver=solver,
+                             nstepmax=3000)
+    tp = col.CollapseTableParams(Nx=shape[0], Ny=shape[1], Nz=shape[2])
+    t = col.make_table(ep, tp)
+    x1, x2, y1, y2, z1, z2 = tp.axes
+    X = x1 + np.arange(tp.Nx) * ((x2 - x1) / (tp.Nx - 1))
+    Y = y1 + np.arange(tp.Ny) * ((y2 - y1) / (tp.Ny - 1))
+    Z = z1 + np.arange(tp.Nz) * ((z2 - z1) / (tp.Nz - 1))
+    import math
+    F = np.array([math.pow(10.0, x) for x in X])
+    k, j, i = np.meshgrid(np.arange(tp.Nz), np.arange(tp.Ny), np.arange(tp.Nx), indexing="ij")
+    z, _, _ = col.evolve_ellipses(F[i.ravel()], Y[j.ravel()], (Z[k] * Y[j]).ravel(), ep)
+    assert np.array_equal(t.ravel(), z.cpu().numpy().astype(np.float32))
