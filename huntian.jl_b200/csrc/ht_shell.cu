@@ -6,8 +6,8 @@
 // outward (the per-shell gather of ShellAnalysisGPU.jl:153-229 / ext/CUDAExt.jl:752-924):
 // each lane accumulates 13 sums per shell in FP64 from the FP32 cell values (delta,
 // delta*d, delta^T*d, and the symmetrised strain psi_L d_K + psi_K d_L, every product
-// exact in FP64); the lanes' partial sums are combined in FP64 in a fixed order through
-// shared memory, and the shell's profile (Fbar, gradients, strain) goes to a per-group
+// exact in FP64); the lanes' partial sums are combined in FP64 in a fixed order by
+// exchanges, and the shell's profile (Fbar, gradients, strain) goes to a per-group
 // scratch slot in FP64.  The walk stops as
 // soon as every shell the post-processing reads has been gathered.  The same group then
 // runs the post-processing of RadialShell.jl:449-859 / ext/CUDAExt.jl:1213-1912 in FP64:
@@ -53,10 +53,19 @@ enum : int {
 static_assert(P_SR % 4 == 0 && P_G == P_SR + 6 && P_GF == P_G + 3 && P_GF + 3 == kRec,
               "SR, G, Gf: twelve contiguous doubles on a 32-byte boundary at the row's end");
 
-// Shared-memory staging per group: [G + 1][kStepW] doubles for inward-walk steps.
+// Shared-memory staging per group: [G + 1][kStepW] doubles for inward-walk steps, or, where
+// the lanes combine through it, [kSums][G + 1] doubles for a shell's partial sums (and room
+// that sets neighbouring groups half the banks apart).
 constexpr int kStepW = 8;       // an inward step's strain, eigen trace and zvir
-__host__ __device__ constexpr int group_smem_doubles(int G) { return (G + 1) * kStepW; }
-constexpr int kWarpSmemDoubles = kPeaksPerItem * group_smem_doubles(kSmallG);
+constexpr int kSums = 14;
+template <bool kExchange>
+__host__ __device__ constexpr int group_smem_doubles(int G) {
+    return kExchange ? (G + 1) * kStepW : kSums * (G + 1) + 10;
+}
+static_assert(group_smem_doubles<false>(kSmallG) >= group_smem_doubles<true>(kSmallG) &&
+                  group_smem_doubles<false>(kSmallG) % 16 == 8, "steps fit; half the banks");
+template <bool kExchange>
+constexpr int kWarpSmemDoubles = kPeaksPerItem * group_smem_doubles<kExchange>(kSmallG);
 
 struct WalkArgs {
     const float4* rec;
@@ -211,19 +220,37 @@ __device__ __forceinline__ Window window_of(const int32_t* __restrict__ wrow,
     return Window{max(f, lo), min(f + (e1 - e0) - 1, hi), wts + e0 - f};
 }
 
-// v[i] summed over the 8 lanes of a group, lane t ending with the sums 2 t and 2 t + 1: at
-// each of three exchanges a lane keeps half of its values and hands the other half to its
-// partner (14 exchanges of 64 bits for 16 values).
-__device__ __forceinline__ void reduce_scatter(const Group& g, double (&v)[16]) {
+// A profile row's values v[i] (v[2] and v[3] unused) summed over the 8 lanes of a group,
+// lane t ending with the sums 2 t and 2 t + 1 in v[0] and v[1]; always the sum
+// ((0 + 4) + (2 + 6)) + ((1 + 5) + (3 + 7)) of the lanes' values.
+//
+// kExchange: at each of three exchanges a lane keeps half of its values and hands the other
+// half to its partner.  Else through shared memory R.  With two blocks per SM the exchange is
+// the faster form, with three shared memory (2.2 M peaks of a 620^3 tile: 30.0 ms against
+// 31.9; 30.8 with sums by lane order, totals read back and groups on the same banks).
+template <bool kExchange>
+__device__ __forceinline__ void combine(const Group& g, double (&v)[16], double* R) {
     static_assert(kSmallG == 8, "three exchanges");
+    if constexpr (kExchange) {
 #pragma unroll
-    for (int half = 8; half >= 2; half >>= 1) {
-        const bool hi = (g.t & (half >> 1)) != 0;
+        for (int half = 8; half >= 2; half >>= 1) {
+            const bool hi = (g.t & (half >> 1)) != 0;
 #pragma unroll
-        for (int i = 0; i < half; ++i) {
-            const double give = hi ? v[i] : v[i + half], keep = hi ? v[i + half] : v[i];
-            v[i] = keep + __shfl_xor_sync(g.mask, give, half >> 1, kSmallG);
+            for (int i = 0; i < half; ++i) {
+                const double give = hi ? v[i] : v[i + half], keep = hi ? v[i + half] : v[i];
+                v[i] = keep + __shfl_xor_sync(g.mask, give, half >> 1, kSmallG);
+            }
         }
+    } else {
+        constexpr int RP = kSmallG + 1;
+#pragma unroll
+        for (int i = 0; i < kSums; ++i) R[i * RP + g.t] = v[i < 2 ? i : i + 2];
+        g.sync();
+        const double* r = R + (g.t == 0 ? 0 : 2 * g.t - 2) * RP;   // lane 1: nothing of its own
+#pragma unroll
+        for (int i = 0; i < 2; ++i, r += RP)
+            v[i] = ((r[0] + r[4]) + (r[2] + r[6])) + ((r[1] + r[5]) + (r[3] + r[7]));
+        g.sync();
     }
 }
 
@@ -666,7 +693,7 @@ __device__ __forceinline__ void count_reject(unsigned* rej, const Group& g, int 
     if (g.t == 0) atomicAdd(rej + r, 1u);
 }
 
-template <bool PACKED>
+template <bool PACKED, bool kExchange>
 __device__ __forceinline__ void process_peak(const WalkArgs& a, long long p, double* __restrict__ P,
                              double* __restrict__ R, const Group& g, unsigned* rej) {
     const double* rad = a.rad;
@@ -730,9 +757,7 @@ __device__ __forceinline__ void process_peak(const WalkArgs& a, long long p, dou
             acc[12].add_prod(e1, d2); acc[12].add_prod(e2, d1);
         });
         // combine the lanes in FP64, in the order of the profile row: delta and the count in
-        // the places of Fbar and the Srb numerator, then SR, G, Gf.   (By exchange: through
-        // shared memory, 14 stores and 16 loads of 64 bits per lane with conflicts, it took a
-        // third of the walk's L1 wavefronts and two barriers.)
+        // the places of Fbar and the Srb numerator, then SR, G, Gf
         double v[16];
         v[0] = acc[0].value();
         v[1] = (double)nin;
@@ -742,7 +767,7 @@ __device__ __forceinline__ void process_peak(const WalkArgs& a, long long p, dou
             v[P_SR + i] = acc[7 + i].value();
             v[P_G + i] = acc[1 + i].value();
         }
-        reduce_scatter(g, v);           // lane t: row values 2 t, 2 t + 1 in v[0], v[1]
+        combine<kExchange>(g, v, R);    // lane t: row values 2 t, 2 t + 1 in v[0], v[1]
         const double Fs = __shfl_sync(g.mask, v[0], 0, kSmallG);
         const double ns = __shfl_sync(g.mask, v[1], 0, kSmallG);
         // finalise shell s (ShellAnalysisGPU.jl:197-228)
@@ -1084,7 +1109,7 @@ __device__ __forceinline__ void process_peak(const WalkArgs& a, long long p, dou
 
 // One work item: kPeaksPerItem consecutive entries of the processing order, one per
 // group of kSmallG lanes; group q of warp w owns scratch slot kPeaksPerItem w + q.
-template <bool PACKED>
+template <bool PACKED, bool kExchange>
 __device__ __forceinline__ void process_item(const WalkArgs& a, long long item, double* P0,
                                              double* W, int lane, unsigned* rej) {
     const int q = lane / kSmallG;
@@ -1096,13 +1121,13 @@ __device__ __forceinline__ void process_item(const WalkArgs& a, long long item, 
     }
     const Group g{kSmallG, lane % kSmallG, q, ((1u << kSmallG) - 1u) << (q * kSmallG)};
     if (p >= 0)
-        process_peak<PACKED>(a, p, P0 + q * a.scratch_stride,
-                             W + q * group_smem_doubles(kSmallG), g, rej);
+        process_peak<PACKED, kExchange>(a, p, P0 + q * a.scratch_stride,
+                             W + q * group_smem_doubles<kExchange>(kSmallG), g, rej);
     __syncwarp();
 }
 
 // BPSM blocks per SM.  With 3 (80 registers, some spills) the walk of 2.2 M peaks of a 620^3
-// tile takes 31.9 ms, with 2 (128 registers, no spills) 32.4; but small batches end on the
+// tile takes 30.0 ms, with 2 (128 registers, no spills) 32.4; but small batches end on the
 // chains of their longest walks, which 2 make shorter: 140,000 peaks 4.31 against 4.69 ms,
 // 40,000 peaks 1.57 against 1.69, 200 peaks 0.33 against 0.39.  Below kFewPeaks the packed
 // walk takes 2.
@@ -1114,7 +1139,8 @@ __global__ void __launch_bounds__(kThreads, BPSM) walk_kernel(const WalkArgs a) 
     if (threadIdx.x < HT_REJECT_COUNT) rej[threadIdx.x] = 0u;
     __syncthreads();
     const int lane = threadIdx.x & 31;
-    double* W = smem + (threadIdx.x >> 5) * kWarpSmemDoubles;
+    constexpr bool kExchange = BPSM == 2;
+    double* W = smem + (threadIdx.x >> 5) * kWarpSmemDoubles<kExchange>;
     const long long gw = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const long long nw = (long long)gridDim.x * kWarpsPerBlock;
     double* P0 = a.scratch + gw * (32 / kSmallG) * a.scratch_stride;
@@ -1128,7 +1154,7 @@ __global__ void __launch_bounds__(kThreads, BPSM) walk_kernel(const WalkArgs a) 
         item = gw;
     }
     while (item < nitems) {
-        process_item<PACKED>(a, item, P0, W, lane, rej);
+        process_item<PACKED, kExchange>(a, item, P0, W, lane, rej);
         if (a.dynamic) {
             int q = 0;
             if (lane == 0) q = atomicAdd(a.queue, 1);
@@ -1312,13 +1338,14 @@ static void fill_args(WalkArgs& a, const ht_ctx* ctx, const ht_fields& f, const 
     a.ntile = (long long)f.n1 * f.n2 * f.n3; a.ncells = ctx->ncells;
 }
 
-static size_t walk_smem_bytes() {
-    return (size_t)kWarpsPerBlock * kWarpSmemDoubles * sizeof(double);
+static size_t walk_smem_bytes(int bpsm) {
+    return (size_t)kWarpsPerBlock *
+           (bpsm == 2 ? kWarpSmemDoubles<true> : kWarpSmemDoubles<false>) * sizeof(double);
 }
 
 template <bool PACKED, int BPSM>
 static int walk_blocks_per_sm(int* bpsm) {
-    const size_t smem = walk_smem_bytes();
+    const size_t smem = walk_smem_bytes(BPSM);
     cudaError_t e = cudaFuncSetAttribute(walk_kernel<PACKED, BPSM>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess)
@@ -1418,7 +1445,7 @@ int ht_launch_walk(ht_ctx* ctx, const ht_peak_batch* b, double alatt, double rma
     HT_CUDA_TRY(cudaMemsetAsync(ctx->d_queue, 0, sizeof(int32_t), st), "queue reset");
     HT_CUDA_TRY(cudaMemsetAsync(ctx->d_stats, 0, 2 * sizeof(unsigned long long), st),
                 "stats reset");
-    const size_t smem = walk_smem_bytes();
+    const size_t smem = walk_smem_bytes(packed && few ? 2 : 3);
     if (!packed) walk_kernel<false, 3><<<(unsigned)blocks, kThreads, smem, st>>>(a);
     else if (few) walk_kernel<true, 2><<<(unsigned)blocks, kThreads, smem, st>>>(a);
     else walk_kernel<true, 3><<<(unsigned)blocks, kThreads, smem, st>>>(a);
@@ -1525,7 +1552,7 @@ extern "C" HT_API int ht_shell_analyse_static(ht_ctx* ctx, const ht_fields* f,
     a.scratch = (double*)scratch; a.scratch_stride = stride;
     a.queue = nullptr; a.dynamic = 0;   // static item-to-warp schedule: no counter to clear
     a.stats = nullptr;
-    const size_t smem = walk_smem_bytes();
+    const size_t smem = walk_smem_bytes(3);
     walk_kernel<false, 3><<<(unsigned)blocks, kThreads, smem, (cudaStream_t)stream>>>(a);
     HT_CUDA_TRY(cudaGetLastError(), "walk_kernel launch (static scratch)");
     ctx->last_kernels = 1;
