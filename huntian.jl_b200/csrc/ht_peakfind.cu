@@ -22,6 +22,8 @@
 //   4. emit  : each segment re-reads its words, ranks its set bits in scan order and
 //              writes (i, j, k, delta_s, lapd_s, filter) plus mask = 1 for every slot
 //              below max_peaks.
+// On small grids (kSmallWords) one launch takes the place of the last three: every CTA
+// counts the words before its own itself.
 // Result: the same peak list, in the same order, as the CPU scan, independent of
 // thread timing (the reference GPU kernel reserves slots with an atomic counter and is
 // order-nondeterministic, ext/CUDAExt.jl:2921).
@@ -43,6 +45,10 @@ constexpr int kWordsPerThread = kSegWords / kEmitThreads;
 struct PfGeom {
     int n, nbuff, inner, wpr;   // words per row = ceil(inner/32)
     long long nwords;           // inner * inner * wpr
+    // small grids (else null): the first block of the flag kernel leaves the running count
+    // here, where pf_emit_small_kernel reads it while its last block advances the count
+    const int64_t* count;
+    int64_t* base;
 };
 
 __global__ void __launch_bounds__(kTX * kTY) pf_flag_kernel(const float* __restrict__ ds,
@@ -58,6 +64,7 @@ __global__ void __launch_bounds__(kTX * kTY) pf_flag_kernel(const float* __restr
     const int i = ib + tx, j = jb + ty;
     const bool active = i < hi && j < hi;
     const long long n = g.n, nn = n * n;
+    if (g.base && tx + ty + blockIdx.x + blockIdx.y + blockIdx.z == 0) *g.base = *g.count;
     const int kend = min(kb + kKZ, hi);
 
     auto load_plane = [&](int slot, int k) {
@@ -171,6 +178,7 @@ __global__ void __launch_bounds__(kTX * kTY) pf_flag_tma_kernel(
     long long word = ((long long)(kb - g.nbuff) * g.inner + (j0 - g.nbuff)) * g.wpr + blockIdx.x;
     const long long word_step_k = (long long)g.inner * g.wpr;
 
+    if (g.base && tid + blockIdx.x + blockIdx.y + blockIdx.z == 0) *g.base = *g.count;
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_addr(&full[s])));
@@ -347,31 +355,45 @@ __global__ void __launch_bounds__(1024) pf_scan_kernel(const int32_t* __restrict
     }
 }
 
-__global__ void __launch_bounds__(kEmitThreads) pf_emit_kernel(
-    const uint32_t* __restrict__ bits, PfGeom g, const int64_t* __restrict__ segbase,
-    const float* __restrict__ ds, const float* __restrict__ lapd_s, int8_t* __restrict__ mask,
-    int32_t filter_idx, int64_t max_peaks, ht_peaks out, int32_t* status) {
-    __shared__ int warp_tot[kEmitThreads / 32];
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const long long w0 = (long long)blockIdx.x * kSegWords + (long long)tid * kWordsPerThread;
-    const long long seg0 = __ldg(segbase + blockIdx.x);   // in flight with the words
-    uint32_t words[kWordsPerThread];
-    static_assert(kWordsPerThread == 8, "two 16-byte loads per thread");
-    if (w0 + kWordsPerThread <= g.nwords) {
-        // 32-byte aligned: the workspace is, and w0 is a multiple of 8 words
-        const uint4 a = __ldg(reinterpret_cast<const uint4*>(bits + w0));
-        const uint4 b = __ldg(reinterpret_cast<const uint4*>(bits + w0 + 4));
-        words[0] = a.x; words[1] = a.y; words[2] = a.z; words[3] = a.w;
-        words[4] = b.x; words[5] = b.y; words[6] = b.z; words[7] = b.w;
-    } else {
-#pragma unroll
-        for (int t = 0; t < kWordsPerThread; ++t)
-            words[t] = w0 + t < g.nwords ? bits[w0 + t] : 0u;
+// Where the peaks go, and what a thread does with the set bits of word w from `slot` on.
+struct PfEmit {
+    PfGeom g;
+    const float* ds;
+    const float* lapd_s;
+    int8_t* mask;
+    int32_t filter_idx;
+    int64_t max_peaks;
+    ht_peaks out;
+    int32_t* status;
+};
+__device__ __forceinline__ void pf_emit_word(const PfEmit& a, uint32_t wd, long long w,
+                                             long long& slot) {
+    const PfGeom& g = a.g;
+    const long long n = g.n, nn = n * n;
+    const long long row = w / g.wpr;
+    const int ib = (int)(w - row * g.wpr) * 32;
+    const int kk = (int)(row / g.inner), jj = (int)(row - (long long)kk * g.inner);
+    while (wd) {
+        const int b = __ffs(wd) - 1;
+        wd &= wd - 1;
+        if (slot >= a.max_peaks) return;
+        const int i = g.nbuff + ib + b, j = g.nbuff + jj, k = g.nbuff + kk;   // 0-based
+        const long long cidx = (long long)i + n * j + nn * k;
+        if (!HT_INDEX_OK(a.status, cidx, nn * n)) continue;
+        a.out.i[slot] = i + 1;
+        a.out.j[slot] = j + 1;
+        a.out.k[slot] = k + 1;
+        a.out.delta[slot] = a.ds[cidx];
+        if (a.out.lapd) a.out.lapd[slot] = a.lapd_s ? a.lapd_s[cidx] : 0.f;
+        a.out.filter_idx[slot] = a.filter_idx;
+        a.mask[cidx] = 1;
+        ++slot;
     }
-    int c = 0;
-#pragma unroll
-    for (int t = 0; t < kWordsPerThread; ++t) c += __popc(words[t]);
-    // block exclusive scan of c
+}
+
+// Exclusive sum of c over the block's threads, and the block's total.
+__device__ __forceinline__ int block_exclusive(int c, int* warp_tot, int* total) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int x = c;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -380,36 +402,75 @@ __global__ void __launch_bounds__(kEmitThreads) pf_emit_kernel(
     }
     if (lane == 31) warp_tot[wid] = x;
     __syncthreads();
-    int wbase = 0;
-    for (int i = 0; i < wid; ++i) wbase += warp_tot[i];
-    long long slot = seg0 + wbase + x - c;
-    if (c == 0 || slot >= max_peaks) return;
-    const long long n = g.n, nn = n * n;
+    int wbase = 0, all = 0;
 #pragma unroll
-    for (int t = 0; t < kWordsPerThread; ++t) {
-        uint32_t wd = words[t];
-        if (!wd) continue;
-        const long long w = w0 + t;
-        const long long row = w / g.wpr;
-        const int ib = (int)(w - row * g.wpr) * 32;
-        const int kk = (int)(row / g.inner), jj = (int)(row - (long long)kk * g.inner);
-        while (wd) {
-            const int b = __ffs(wd) - 1;
-            wd &= wd - 1;
-            if (slot >= max_peaks) return;
-            const int i = g.nbuff + ib + b, j = g.nbuff + jj, k = g.nbuff + kk;   // 0-based
-            const long long cidx = (long long)i + n * j + nn * k;
-            if (!HT_INDEX_OK(status, cidx, nn * n)) continue;
-            out.i[slot] = i + 1;
-            out.j[slot] = j + 1;
-            out.k[slot] = k + 1;
-            out.delta[slot] = ds[cidx];
-            if (out.lapd) out.lapd[slot] = lapd_s ? lapd_s[cidx] : 0.f;
-            out.filter_idx[slot] = filter_idx;
-            mask[cidx] = 1;
-            ++slot;
-        }
+    for (int i = 0; i < kEmitThreads / 32; ++i) {
+        if (i < wid) wbase += warp_tot[i];
+        all += warp_tot[i];
     }
+    *total = all;
+    return wbase + x - c;
+}
+
+__global__ void __launch_bounds__(kEmitThreads) pf_emit_kernel(const uint32_t* __restrict__ bits,
+                                                               const int64_t* __restrict__ segbase,
+                                                               const PfEmit a) {
+    __shared__ int warp_tot[kEmitThreads / 32];
+    const long long w0 = (long long)blockIdx.x * kSegWords +
+                         (long long)threadIdx.x * kWordsPerThread;
+    const long long seg0 = __ldg(segbase + blockIdx.x);   // in flight with the words
+    uint32_t words[kWordsPerThread];
+    static_assert(kWordsPerThread == 8, "two 16-byte loads per thread");
+    if (w0 + kWordsPerThread <= a.g.nwords) {
+        // 32-byte aligned: the workspace is, and w0 is a multiple of 8 words
+        const uint4 p = __ldg(reinterpret_cast<const uint4*>(bits + w0));
+        const uint4 q = __ldg(reinterpret_cast<const uint4*>(bits + w0 + 4));
+        words[0] = p.x; words[1] = p.y; words[2] = p.z; words[3] = p.w;
+        words[4] = q.x; words[5] = q.y; words[6] = q.z; words[7] = q.w;
+    } else {
+#pragma unroll
+        for (int t = 0; t < kWordsPerThread; ++t)
+            words[t] = w0 + t < a.g.nwords ? bits[w0 + t] : 0u;
+    }
+    int c = 0, total;
+#pragma unroll
+    for (int t = 0; t < kWordsPerThread; ++t) c += __popc(words[t]);
+    long long slot = seg0 + block_exclusive(c, warp_tot, &total);
+    if (c == 0 || slot >= a.max_peaks) return;
+#pragma unroll
+    for (int t = 0; t < kWordsPerThread; ++t)
+        if (words[t]) pf_emit_word(a, words[t], w0 + t, slot);
+}
+
+// Count, scan and emit of a small grid in one launch: a CTA takes 256 words, one per thread,
+// and adds up the words before them itself (at most 256 KB from L2).  Three launches are
+// bound by their own latency there (2.7 + 3.3 + 5.2 us on a 128^3 region, 8 words in a row
+// per emitting thread; this one 9.4 us, and on a 48^3 region 3.8 against 13.8).  Counting
+// takes over above that size: the words before a CTA's grow with the square of the words.
+constexpr long long kSmallWords = 1 << 16;
+__global__ void __launch_bounds__(kEmitThreads) pf_emit_small_kernel(
+    const uint32_t* __restrict__ bits, const PfEmit a, int64_t* count, int64_t* found) {
+    __shared__ int warp_tot[kEmitThreads / 32], warp_before[kEmitThreads / 32];
+    const int tid = threadIdx.x;
+    const int first = blockIdx.x * kEmitThreads, w = first + tid;
+    const uint32_t word = w < a.g.nwords ? __ldg(bits + w) : 0u;
+    int s = 0, before, total;
+    const uint4* b4 = reinterpret_cast<const uint4*>(bits);   // first is a multiple of 4 words
+#pragma unroll 4
+    for (int x = tid; x < first / 4; x += kEmitThreads) {
+        const uint4 p = __ldg(b4 + x);
+        s += __popc(p.x) + __popc(p.y) + __popc(p.z) + __popc(p.w);
+    }
+    block_exclusive(s, warp_before, &before);
+    const int excl = block_exclusive(__popc(word), warp_tot, &total);
+    const long long base = *a.g.base;
+    long long slot = base + before + excl;
+    if (tid == 0 && blockIdx.x == gridDim.x - 1) {
+        const long long all = before + total;
+        if (found) *found += all;
+        *count = base + all < a.max_peaks ? base + all : a.max_peaks;
+    }
+    if (word && slot < a.max_peaks) pf_emit_word(a, word, w, slot);
 }
 
 
@@ -455,6 +516,8 @@ int ht_launch_peakfind(ht_ctx* ctx, const float* d_delta_s, const float* d_lapd_
     g.inner = n - 2 * nbuff;
     g.wpr = (g.inner + 31) / 32;
     g.nwords = (long long)g.inner * g.inner * g.wpr;
+    g.count = out->count;
+    g.base = nullptr;
     ctx->last_kernels = 0;
     if (g.inner <= 0) return HT_OK;
     const long long nseg = (g.nwords + kSegWords - 1) / kSegWords;
@@ -465,6 +528,8 @@ int ht_launch_peakfind(ht_ctx* ctx, const float* d_delta_s, const float* d_lapd_
     uint32_t* bits = (uint32_t*)ctx->d_pf_ws;
     int64_t* segbase = (int64_t*)((char*)ctx->d_pf_ws + bits_bytes);
     int32_t* segcount = (int32_t*)(segbase + nseg);
+    const bool small = g.nwords <= kSmallWords;
+    if (small) g.base = segbase;
 
     const unsigned gx = (unsigned)((g.inner + kTX - 1) / kTX);
     const unsigned gy = (unsigned)((g.inner + kTY - 1) / kTY);
@@ -486,15 +551,21 @@ int ht_launch_peakfind(ht_ctx* ctx, const float* d_delta_s, const float* d_lapd_
         pf_flag_kernel<<<grid1, dim3(kTX, kTY), 0, st>>>(d_delta_s, d_mask, g, fcrit, bits);
         HT_CUDA_TRY(cudaGetLastError(), "pf_flag_kernel launch");
     }
+    const PfEmit e{g, d_delta_s, d_lapd_s, d_mask, filter_idx, max_peaks, *out,
+                   ht_status_word(ctx)};
+    if (small) {
+        pf_emit_small_kernel<<<(unsigned)((g.nwords + kEmitThreads - 1) / kEmitThreads),
+                               kEmitThreads, 0, st>>>(bits, e, out->count, out->found);
+        HT_CUDA_TRY(cudaGetLastError(), "pf_emit_small_kernel launch");
+        ctx->last_kernels = 2;
+        return HT_OK;
+    }
     pf_count_kernel<<<(unsigned)nseg, kEmitThreads, 0, st>>>(bits, g.nwords, segcount);
     HT_CUDA_TRY(cudaGetLastError(), "pf_count_kernel launch");
     pf_scan_kernel<<<1, 1024, 0, st>>>(segcount, (int)nseg, segbase, out->count, out->found,
                                        max_peaks);
     HT_CUDA_TRY(cudaGetLastError(), "pf_scan_kernel launch");
-    pf_emit_kernel<<<(unsigned)nseg, kEmitThreads, 0, st>>>(bits, g, segbase, d_delta_s,
-                                                             d_lapd_s, d_mask, filter_idx,
-                                                             max_peaks, *out,
-                                                             ht_status_word(ctx));
+    pf_emit_kernel<<<(unsigned)nseg, kEmitThreads, 0, st>>>(bits, segbase, e);
     HT_CUDA_TRY(cudaGetLastError(), "pf_emit_kernel launch");
     ctx->last_kernels = 4;
     return HT_OK;

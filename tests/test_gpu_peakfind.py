@@ -314,3 +314,14 @@ def test_smooth_tile_planes(ht, finder, n, lo, hi):
     scale = np.abs(full).max()
     assert np.abs(part[lo:hi] - full[lo:hi]).max() <= 1e-6 * scale
 
+
+
+@pytest.mark.parametrize("n,nbuff", [(5, 2), (12, 1), (43, 5), (138, 5), (139, 5)])
+@pytest.mark.parametrize("cap", [1 << 20, 700])
+def test_single_launch_emit_edges(ht, oracle, finder, n, nbuff, cap):
+    """One word, part of a 256-word CTA, CTAs that count others' words, the largest grid with
+    the single-launch emit (128^3 inner cells: 65,536 words) and the smallest without; two
+    fields with the count and the mask carried, and lists cut off inside a CTA's words."""
+    rng = np.random.default_rng(n)
+    fields = [rng.standard_normal((n, n, n)).astype(np.float32) for _ in range(2)]
+    _both(ht, oracle, finder, fields, nbuff, [0.5, 0.2], max_peaks=cap)
