@@ -903,7 +903,9 @@ extern "C" HT_API int ht_evolve_ellipses(int device, const ht_ellipsoid* ep,
     cudaStream_t st = (cudaStream_t)stream;
     // the growth table and the reciprocals of its 4-point windows, in one upload
     const int nt = growth->ntab;
-    std::vector<double> h(growth->atab, growth->atab + nt);
+    std::vector<double> h;
+    h.reserve(15 * (size_t)nt);
+    h.insert(h.end(), growth->atab, growth->atab + nt);
     h.insert(h.end(), growth->D_atab, growth->D_atab + nt);
     h.insert(h.end(), growth->dlnD_dlnatab, growth->dlnD_dlnatab + nt);
     // (while a graph is captured the copies must come from the caller's own arrays, which
@@ -974,14 +976,15 @@ extern "C" HT_API int ht_collapse_table(int device, const ht_ellipsoid* ep,
     // e_v slowest and from its largest value down: the RK4's steps go with e_v first (650 to
     // 10,000 over the default table), so that a warp's entries take about as long, and the
     // long warps start first, each on a scheduler of its own
-    for (long long q = 0; q < n; ++q) {
-        const int i = (int)(q % nx), k = (int)((q / nx) % nz),
-                  j = ny - 1 - (int)(q / ((long long)nx * nz));
-        const double y = Y1 + j * dY, z = Z1 + k * dZ;
-        h[q] = Frho[i];
-        h[n + q] = y;
-        h[2 * n + q] = z * y;
-    }
+    long long q = 0;
+    for (int j = ny - 1; j >= 0; --j)
+        for (int k = 0; k < nz; ++k)
+            for (int i = 0; i < nx; ++i, ++q) {
+                const double y = Y1 + j * dY, z = Z1 + k * dZ;
+                h[q] = Frho[i];
+                h[n + q] = y;
+                h[2 * n + q] = z * y;
+            }
     HT_CUDA_TRY(cudaSetDevice(device), "ht_collapse_table: cudaSetDevice");
     double* d = nullptr;
     HT_CUDA_TRY(cudaMalloc((void**)&d, 4 * (size_t)n * sizeof(double)), "ht_collapse_table: buffers");
@@ -998,9 +1001,10 @@ extern "C" HT_API int ht_collapse_table(int device, const ht_ellipsoid* ep,
     }
     cudaFree(d);
     if (rc != HT_OK) return rc;
-    for (long long q = 0; q < n; ++q) {
-        const long long i = q % nx, k = (q / nx) % nz, j = ny - 1 - q / ((long long)nx * nz);
-        table[i + nx * (j + ny * k)] = (float)h[q];
-    }
+    q = 0;
+    for (int j = ny - 1; j >= 0; --j)
+        for (int k = 0; k < nz; ++k)
+            for (int i = 0; i < nx; ++i, ++q)
+                table[i + (long long)nx * (j + (long long)ny * k)] = (float)h[q];
     return HT_OK;
 }

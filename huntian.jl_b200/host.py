@@ -426,7 +426,9 @@ def peak_find_tile_gpu(delta_tile, filters: Sequence, fcrits: Sequence[float], t
     assert delta.shape == (n, n, n) and len(filters) == len(fcrits)
     if finder is None:
         raise ValueError("pass finder=HaloFinder(...) (the library context)")
-    mask = _dev(tile_masks_in, torch.int8, device).clone()
+    mask = _dev(tile_masks_in, torch.int8, device)
+    if isinstance(tile_masks_in, torch.Tensor):   # host arrays were copied already
+        mask = mask.clone()
     boxsize = n * float(alatt)   # periodic tile: boxsize_local = n * alatt
     has_lapd = ioutshear >= 1
     delta_k = torch.fft.rfftn(delta, dim=(0, 1, 2)).contiguous()
@@ -459,18 +461,18 @@ def peak_find_tile_gpu(delta_tile, filters: Sequence, fcrits: Sequence[float], t
     if return_device:
         res_dev["mask"] = mask
         return res_dev
-    i = sl(out["i"]).cpu().numpy().astype(np.int64)
-    j = sl(out["j"]).cpu().numpy().astype(np.int64)
-    k = sl(out["k"]).cpu().numpy().astype(np.int64)
-    fidx = sl(out["filter_idx"]).cpu().numpy()
-    fdelta = sl(out["delta"]).cpu().numpy()
+    # the lists in one copy (each has a wait of its own), the floats as their bits
+    names = ("i", "j", "k", "filter_idx", "delta") + (("lapd",) if has_lapd else ())
+    lists = torch.stack([sl(out[c]).view(torch.int32) for c in names]).cpu().numpy()
+    i, j, k = (lists[c].astype(np.int64) for c in range(3))
+    fidx, fdelta = lists[3], lists[4].view(np.float32).copy()
     cen = 0.5 * (n + 1)
     Rfs = np.array([float(f[2]) for f in filters], dtype=np.float64)
     Rf_out = Rfs[fidx - 1] if npk else np.zeros(0)
     peaks = PeakCandidate(i, j, k, i + (j - 1) * n + (k - 1) * n * n,
                           xbx + alatt * (i - cen), ybx + alatt * (j - cen),
                           zbx + alatt * (k - cen), fdelta, Rf_out)
-    d2 = sl(out["lapd"]).cpu().numpy() if has_lapd else np.zeros(npk, np.float32)
+    d2 = lists[5].view(np.float32).copy() if has_lapd else np.zeros(npk, np.float32)
     return {"peaks": peaks, "Rf": Rf_out, "FcRf": fdelta, "d2Rf": d2,
             "mask": mask.cpu().numpy()}
 
