@@ -524,10 +524,12 @@ def run_ours(args, rank, world, device):
                      "alg_bytes_per_launch": alg_bytes, "cells_walked": cells},
         # ours per step: per filter the window table (+ its kz rows on the pencil path),
         # 3 transform kernels (pencil passes, or the transposed path's window/transpose
-        # kernels) and 4 peak-scan kernels; per step the pencil transpose, pack, order keys,
+        # kernels) and 4 peak-scan kernels (2 up to 65,536 bitmap words); per step the pencil transpose, pack, order keys,
         # walk, halo flags and records (+ features and MLP in learned mode); cuFFT and CUB
         # launches not counted
-        "gpu_launches": int(args.steps * ((9 if W.pencil else 8) * nf +
+        "gpu_launches": int(args.steps * (((9 if W.pencil else 8) -
+                                           (2 if W.n * W.n * -(-W.n // 32) <= 65536 else 0)) *
+                                          nf +
                                           (1 if W.pencil else 0) + 5 +
                                           (2 if args.mode == "learned" else 0))),
         "clocks": ck,
