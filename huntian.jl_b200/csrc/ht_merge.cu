@@ -142,9 +142,10 @@ struct Nbr {
     const int32_t* at;         // rank -> place in cell order
 };
 
-// Cell rows that can hold a point within `reach` of v (every point whose distance, as dist3
+// Cell rows that can hold a point within `reach` > 0 of v (every point whose distance, as dist3
 // rounds it, is below reach: the box is wider by more than the roundings of the distance and
-// of its own bounds).
+// of its own bounds).  A negative reach would turn the bounds round, and for_neighbours would
+// take the product of two negative extents for a count of rows, some of them past the table.
 struct Box {
     int x0, x1, y0, y1, z0, z1;
 };
@@ -274,6 +275,7 @@ __global__ void __launch_bounds__(kCta ? kBigThreads : 256) overlap_kernel(
         const float4 v = nb.xyzr[s];
         if (!kCta && v.w > nb.big) return;
         const double rq = v.w;
+        if (!(rq > 0.0)) return;   // later radii are no larger: no distance is below the sum
         const int rank = nb.rank[s];
         double acc = 0.0;
         for_neighbours<kCta>(nb, box_of(nb.g, v, dmul(2.0, rq)), [&](int p) {

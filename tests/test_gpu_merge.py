@@ -129,6 +129,46 @@ def test_search_sizes_match_oracle(ht, finder, n, lo, hi, span, reduce):
     assert _ulps(got[:, 6], want[:, 6]).max(initial=0) <= 1
 
 
+@pytest.mark.parametrize("reduce", [False, True])
+@pytest.mark.parametrize("low", [0.0, -1.0, -100.0])
+def test_radii_that_cover_nothing(ht, finder, low, reduce):
+    """Zero and negative radii (-1 marks a peak without collapse) among ordinary ones, in the
+    corners of the cell grid too: such halos cover and overlap nothing, and a volume reduction
+    leaves them no volume.  n 2^-53 / (3 s) bounds the radii as in the test above."""
+    rng = np.random.default_rng(17)
+    n = 2000
+    rec = rng.normal(0, 1, (n, 11)).astype(np.float32)
+    rec[:, :3] = rng.uniform(0, 10, (n, 3))
+    rec[:8, :3] = [[10.0 * (c >> d & 1) for d in range(3)] for c in range(8)]
+    rec[:, 6] = np.where(rng.random(n) < 0.4, low, rng.uniform(0.05, 0.4, n))
+    rec[:8, 6] = low
+    got = _merge(ht, finder, rec, volume_reduction=reduce)
+    want = oc.merge_catalog(rec, volume_reduction=reduce)
+    assert got.shape == want.shape and (reduce or (want[:, 6] == low).sum() > 500)
+    other = [c for c in range(11) if c != 6]
+    assert np.array_equal(got[:, other], want[:, other])
+    assert _ulps(got[:, 6], want[:, 6]).max() <= (1 if reduce else 0)
+
+
+@pytest.mark.parametrize("reduce", [False, True])
+def test_nan_radius_leaves_the_others_alone(ht, finder, reduce):
+    """A radius that is not a number is refused or, where the largest radius comes out finite,
+    covers nothing and changes no other halo."""
+    rng = np.random.default_rng(18)
+    rec = rng.normal(0, 1, (3000, 11)).astype(np.float32)
+    rec[:, :3] = rng.uniform(0, 10, (3000, 3))
+    rec[:, 6] = rng.uniform(0.05, 0.4, 3000)
+    rec[1234, 6] = np.nan
+    try:
+        got = _merge(ht, finder, rec, volume_reduction=reduce)
+    except ht.HTError:
+        return
+    got = got[~np.isnan(got[:, 6])]
+    want = oc.merge_catalog(np.delete(rec, 1234, 0), volume_reduction=reduce)
+    assert got.shape == want.shape
+    assert _ulps(got[:, 6], want[:, 6]).max() <= (1 if reduce else 0)
+
+
 @pytest.mark.parametrize("ievol", [0, 1])
 def test_finalize_eulerian_matches_oracle(ht, finder, ievol):
     cat = ht.catalog
