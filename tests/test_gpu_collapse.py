@@ -6,6 +6,11 @@ fixed-step RK4 (EllipsoidalCollapse.jl:149-590, solver = :rk4) and the adaptive 
 Both sides run the same FP64 operations in the same order (the device file is built
 without fused multiply-adds, and the logarithm of the oblate shape branch and the Tsit5
 controller's power are series that both carry), so the values agree to the bit."""
+import dataclasses
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -170,3 +175,103 @@ def test_table_order_and_edges(ht, oracle, solver, shape):
     k, j, i = np.meshgrid(np.arange(tp.Nz), np.arange(tp.Ny), np.arange(tp.Nx), indexing="ij")
     z, _, _ = col.evolve_ellipses(F[i.ravel()], Y[j.ravel()], (Z[k] * Y[j]).ravel(), ep)
     assert np.array_equal(t.ravel(), z.cpu().numpy().astype(np.float32))
+
+
+def _evolve_into(col, ep, args, out):
+    """ht_evolve_ellipses on the current stream into out = (z, D, fc, steps)."""
+    from huntian_b200 import _lib
+    e, gr, keep = ep._structs()
+    C = col.C
+    _lib.check(_lib.load().ht_evolve_ellipses(
+        0, C.byref(e), C.byref(gr), args[0].numel(), *(a.data_ptr() for a in args), 1,
+        *(o.data_ptr() for o in out), torch.cuda.current_stream().cuda_stream))
+    return keep
+
+
+@pytest.mark.parametrize("solver", ["rk4", "diffeq"])
+def test_captured_and_without_reciprocals(ht, planck, solver):
+    """A call under stream capture, and one that does without the reciprocals of the growth
+    table's spacings because one is too small for them (here beyond the range that is used):
+    both give every bit of the ordinary call's results."""
+    cp, g = planck
+    col = ht.collapse
+    rng = np.random.default_rng(5)
+    n = 333
+    F = 10.0 ** rng.uniform(np.log10(1.2), np.log10(9.0), n)
+    e = rng.uniform(0.0, 0.5, n)
+    args = [torch.as_tensor(v, device="cuda") for v in (F, e, rng.uniform(-1, 1, n) * e)]
+    ep = col.EllipsoidParams(cp, dlin_tables=g, solver=solver, nstepmax=3000)
+    want = col.evolve_ellipses(*args, ep, steps=True)
+    assert (want[0] > 0).sum() > n // 2
+
+    out = [torch.zeros_like(w) for w in want]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        keep = _evolve_into(col, ep, args, out)
+    graph.replay()
+    torch.cuda.synchronize()
+    del keep, graph
+    for a, b in zip(out, want):
+        assert torch.equal(a, b)
+
+    more = lambda t, last: np.r_[t, last]                       # noqa: E731
+    g2 = dataclasses.replace(g, atab=more(g.atab, g.atab[-1] + 5e-13),
+                             D_atab=more(g.D_atab, g.D_atab[-1]),
+                             dlnD_dlnatab=more(g.dlnD_dlnatab, g.dlnD_dlnatab[-1]))
+    assert 0 < g2.atab[-1] - g2.atab[-2] < 1e-12 and g.amaxtab <= g.atab[-1]
+    got = col.evolve_ellipses(*args, col.EllipsoidParams(cp, dlin_tables=g2, solver=solver,
+                                                         nstepmax=3000), steps=True)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
+_NO_NEW = """
+#include <cstdlib>
+#include <new>
+static std::size_t limit = 0;
+extern "C" void refuse_from(std::size_t n) { limit = n; }
+void* operator new(std::size_t n) {
+    if (limit && n >= limit) throw std::bad_alloc();
+    if (void* p = malloc(n ? n : 1)) return p;
+    throw std::bad_alloc();
+}
+void operator delete(void* p) noexcept { free(p); }
+void operator delete(void* p, std::size_t) noexcept { free(p); }
+"""
+
+
+def _child_without_memory(shim, path):
+    import ctypes
+    from conftest import load_package
+    ht = load_package()
+    col = ht.collapse
+    refuse = ctypes.CDLL(shim).refuse_from
+    refuse.argtypes = [ctypes.c_size_t]
+    ep = col.EllipsoidParams(ht.catalog.CosmologyParams(Om=0.315, OL=0.685), solver="rk4")
+    args = [torch.tensor(v, dtype=torch.float64, device="cuda")
+            for v in ([2.0, 3.0], [0.1, 0.3], [0.0, 0.1])]
+    out = [torch.zeros(2, dtype=t, device="cuda") for t in (torch.float64,) * 3 + (torch.int32,)]
+    _evolve_into(col, ep, args, out)       # the driver's own first-use allocations
+    out[0].zero_()
+    refuse(16384)
+    _evolve_into(col, ep, args, out)
+    refuse(0)
+    np.save(path, out[0].cpu().numpy())
+
+
+def test_host_memory_refused(ht, tmp_path):
+    """A host that has no memory left (operator new refuses 16 KB and more while the call runs,
+    in a child process) is no reason for ht_evolve_ellipses to end the program."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    src, so, out = (str(tmp_path / f) for f in ("no.cpp", "no.so", "z.npy"))
+    with open(src, "w") as f:
+        f.write(_NO_NEW)
+    subprocess.run(["g++", "-O1", "-shared", "-fPIC", src, "-o", so], check=True)
+    code = (f"import sys; sys.path.insert(0, {here!r}); import conftest; "
+            f"import test_gpu_collapse as t; t._child_without_memory({so!r}, {out!r})")
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=here, timeout=600,
+                   env=dict(os.environ, LD_PRELOAD=so))
+    col = ht.collapse
+    ep = col.EllipsoidParams(ht.catalog.CosmologyParams(Om=0.315, OL=0.685), solver="rk4")
+    want = col.evolve_ellipses([2.0, 3.0], [0.1, 0.3], [0.0, 0.1], ep)[0].cpu().numpy()
+    assert np.array_equal(np.load(out), want) and (want > 0).all()
