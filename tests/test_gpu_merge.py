@@ -129,6 +129,18 @@ def test_search_sizes_match_oracle(ht, finder, n, lo, hi, span, reduce):
     assert _ulps(got[:, 6], want[:, 6]).max(initial=0) <= 1
 
 
+@pytest.mark.parametrize("n", [2, 3, 5, 9, 127, 128])
+def test_chains_of_every_length(ht, finder, n):
+    """Chains in which each halo covers the next one and nothing else: one is decided a round,
+    n rounds, with the host looking at every round (below 128 halos) and at every fourth."""
+    rec = np.zeros((n, 11), np.float32)
+    r = 4.0 * 0.999 ** np.arange(n)
+    rec[:, 0] = np.r_[0.0, np.cumsum(0.9 * r[:-1])]
+    rec[:, 6] = r
+    got = _merge(ht, finder, rec)
+    assert np.array_equal(got, oc.merge_catalog(rec)) and got.shape[0] == (n + 1) // 2
+
+
 @pytest.mark.parametrize("reduce", [False, True])
 @pytest.mark.parametrize("low", [0.0, -1.0, -100.0])
 def test_radii_that_cover_nothing(ht, finder, low, reduce):
