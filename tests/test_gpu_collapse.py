@@ -157,24 +157,17 @@ def test_tsit5_table_and_events_match_oracle(ht, planck):
 
 @pytest.mark.parametrize("solver", ["rk4", "diffeq"])
 @pytest.mark.parametrize("shape", [(2, 2, 2), (33, 2, 3), (5, 31, 2)])
-def test_table_order_and_edges(ht, oracle, solver, shape):
-    """Tables whose entries do not fill the last warp, at the extremes of the axes: shapes near
-    the spherical limit (e_v = 0), oblate and prolate ones (p_v / e_v = -1, 1) and radii past
-    the division-free form of the shape integrals' test.  Every entry equals the scalar call."""
+def test_table_order_and_edges(ht, planck, solver, shape):
+    """Tables whose entries do not fill the last warp, at the extremes of the axes: the
+    spherical limit (e_v = 0), oblate and prolate shapes (p_v / e_v = -1, 1) and the largest
+    e_v.  Every entry is the oracle's (the host's sqrt and division round as the operators
+    that the device's forms stand for) and sits at its place in the table."""
+    cp, g = planck
     col = ht.collapse
-    ep = col.EllipsoidParams(ht.catalog.CosmologyParams(Om=0.3, OL=0.7), solver=solver,
-                             nstepmax=3000)
-    tp = col.CollapseTableParams(Nx=shape[0], Ny=shape[1], Nz=shape[2])
-    t = col.make_table(ep, tp)
-    x1, x2, y1, y2, z1, z2 = tp.axes
-    X = x1 + np.arange(tp.Nx) * ((x2 - x1) / (tp.Nx - 1))
-    Y = y1 + np.arange(tp.Ny) * ((y2 - y1) / (tp.Ny - 1))
-    Z = z1 + np.arange(tp.Nz) * ((z2 - z1) / (tp.Nz - 1))
-    import math
-    F = np.array([math.pow(10.0, x) for x in X])
-    k, j, i = np.meshgrid(np.arange(tp.Nz), np.arange(tp.Ny), np.arange(tp.Nx), indexing="ij")
-    z, _, _ = col.evolve_ellipses(F[i.ravel()], Y[j.ravel()], (Z[k] * Y[j]).ravel(), ep)
-    assert np.array_equal(t.ravel(), z.cpu().numpy().astype(np.float32))
+    ep = col.EllipsoidParams(cp, dlin_tables=g, solver=solver, nstepmax=3000)
+    t = col.make_table(ep, col.CollapseTableParams(Nx=shape[0], Ny=shape[1], Nz=shape[2]))
+    eo = oc.EllipsoidOracle(g, cp.Om, cp.OL, solver=solver, nstepmax=3000)
+    assert np.array_equal(t, np.transpose(eo.make_table(*shape), (2, 1, 0)))
 
 
 def _evolve_into(col, ep, args, out):
