@@ -1126,12 +1126,14 @@ __device__ __forceinline__ void process_item(const WalkArgs& a, long long item, 
     __syncwarp();
 }
 
-// BPSM blocks per SM.  With 3 (80 registers, some spills) the walk of 2.2 M peaks of a 620^3
-// tile takes 30.0 ms, with 2 (128 registers, no spills) 32.4; but small batches end on the
-// chains of their longest walks, which 2 make shorter: 140,000 peaks 4.31 against 4.69 ms,
-// 40,000 peaks 1.57 against 1.69, 200 peaks 0.33 against 0.39.  Below kFewPeaks the packed
-// walk takes 2.
-constexpr long long kFewPeaks = 500000;
+// BPSM blocks per SM.  Three (80 registers, some spills) have more loads in flight; two (128
+// registers, no spills) make the chains of the longest walks shorter, on which small batches
+// end.  The packed walk takes two below kFewPeaks.  Two against three, ms, every peak of a box
+// in the learned order: with 40 filters and 1.95 Mpc/h cells 86,000 peaks 2.62 and 2.73,
+// 168,000 3.08 and 3.04, 237,000 4.03 and 3.91, 354,000 5.79 and 5.56, 2.8 M 40.6 and 38.5; with
+// 80 filters and 1.46 Mpc/h cells 182,000 peaks 4.85 and 5.10, 231,000 5.07 and 4.83, 748,000
+// 14.5 and 13.6.  (In Morton order the lines lie at 110,000 and 200,000 peaks.)
+constexpr long long kFewPeaks = 180000;
 template <bool PACKED, int BPSM>
 __global__ void __launch_bounds__(kThreads, BPSM) walk_kernel(const WalkArgs a) {
     extern __shared__ double smem[];
@@ -1174,11 +1176,11 @@ __global__ void __launch_bounds__(kThreads, BPSM) walk_kernel(const WalkArgs a) 
 // which then come from L2; in LEARNED mode the four peaks of a warp also walk similar
 // distances.  Walks past kLongWalk cells go first, in the same order among themselves: one
 // of them is a chain of loads up to milliseconds long, and those that came last kept a few
-// warps busy after the others were done (43 % of the SM cycles of a 140,000-peak walk of a
-// 320^3 tile were idle; the walk went from 5.13 to 4.75 ms and that of 40,000 peaks of a
-// 200^3 tile from 1.96 to 1.71; a line at 10 cells was no better, and cost the 2.2 M peaks
-// of a 620^3 tile 2 % in locality).  The order changes no result (outputs are indexed by
-// peak).
+// warps busy after the others were done.  A lower line takes more peaks out of their place: at
+// 12, 16, 24 cells and without a line 150,000 peaks (40 filters, learned order) take 2.60, 2.82,
+// 3.20 and 3.17 ms, 1.2 M 16.4, 16.8, 17.0 and 17.0, 2.8 M 38.9, 38.4, 39.0 and 39.0; 748,000
+// peaks with 80 filters 13.9, 13.6, 15.0 and 15.9.  The order changes no result (outputs are
+// indexed by peak).
 constexpr float kLongWalk = 16.f;
 // The keys are 32 bits wide (four passes of the sort): a long-walk bit over KeyBits.place
 // bits of the Morton code and, in LEARNED mode, kCostBits of cost in 1/16 cells.

@@ -8,8 +8,9 @@ and identical masks.  PLAIN and BATCHED modes must agree bit for bit.
 """
 import numpy as np
 import pytest
+import torch
 
-from gpu_helpers import compare, gpu_find_peaks, run_shell
+from gpu_helpers import compare, gpu_find_peaks, make_box_workload, run_shell
 from test_oracle_golden import FORTRAN, fortran_peak_fields
 
 pytestmark = pytest.mark.gpu
@@ -248,3 +249,28 @@ def test_record_gather_probe(ht, julia_table_path):
     assert np.array_equal(got[ok], want[ok])
     assert np.isnan(got[~ok]).all()
     finder.close()
+
+
+@pytest.mark.parametrize("mode", ["batched", "learned"])
+def test_batch_size_changes_no_result(ht, mode):
+    """Small and large batches run with two and three blocks per SM and combine a group's lanes
+    in two ways: the same peaks five times in one batch give every bit that they give alone."""
+    W = make_box_workload(ht, 128, 250.0, 36, 30, 2.0, 40.0, 12345)
+    f, t, npk = W["finder"], W["tile"], W["npk"]
+    assert 20_000 < npk < 100_000
+    rep = 200_000 // npk + 1
+    f.bind_fields(t["delta"], t["etax"], t["etay"], t["etaz"], t["eta2x"], t["eta2y"],
+                  t["eta2z"], None)
+    cost = torch.rand(npk, device="cuda", generator=torch.Generator("cuda").manual_seed(1)) * 40
+    got = []
+    for k in (1, rep):
+        args = [a.repeat(k) for a in W["args"][:7]] + [W["alatt"]]
+        mask = torch.zeros_like(t["delta"], dtype=torch.int8)
+        res = f.analyse(*args, nbuff=36, mode=mode, mask=mask,
+                        cost=cost.repeat(k) if mode == "learned" else None)
+        torch.cuda.synchronize()
+        got.append({**{c: v.reshape(-1).clone() for c, v in res.items()}, "mask": mask})
+    one, many = got
+    assert torch.equal(one.pop("mask"), many.pop("mask"))
+    for c, v in one.items():
+        assert torch.equal(many[c].view(torch.int32), v.view(torch.int32).repeat(rep)), c
