@@ -1183,20 +1183,21 @@ __global__ void __launch_bounds__(kThreads, BPSM) walk_kernel(const WalkArgs a) 
 // indexed by peak).
 constexpr float kLongWalk = 16.f;
 // The keys are 32 bits wide (four passes of the sort): a long-walk bit over KeyBits.place
-// bits of the Morton code and, in LEARNED mode, kCostBits of cost in 1/16 cells.
+// bits of the Morton code and, in LEARNED mode, KeyBits.cost bits of cost: 1/16 cells in
+// kCostBits, coarser where small blocks leave fewer.
 constexpr int kCostBits = 12;
 struct KeyBits {
     int shift, place;    // Morton bits dropped and kept
-    int total;
+    int cost, total;
 };
 static KeyBits key_bits(int n, int block_bits, bool cost) {
     int nb = 1;
     while (nb < 20 && (1 << nb) < n) ++nb;
-    const int room = 31 - (cost ? kCostBits : 0);
     KeyBits k;
-    k.shift = std::max(cost ? std::min(block_bits, 3 * nb) : 0, 3 * nb - room);
+    k.shift = std::max(cost ? std::min(block_bits, 3 * nb) : 0, 3 * nb - 31);
     k.place = 3 * nb - k.shift;
-    k.total = k.place + 1 + (cost ? kCostBits : 0);
+    k.cost = cost ? std::min(kCostBits, 31 - k.place) : 0;
+    k.total = k.place + 1 + k.cost;
     return k;
 }
 __device__ __forceinline__ unsigned long long spread3(unsigned v) {
@@ -1231,7 +1232,8 @@ __global__ void __launch_bounds__(256) order_key_kernel(const WalkArgs a,
         c = c == c ? fminf(fmaxf(c, 0.f), 1.0e6f) : 0.f;
         reach = c;
         const uint32_t top = (1u << kCostBits) - 1;
-        key = (place << kCostBits) | (top - min((uint32_t)(c * 16.f), top));
+        const uint32_t q = top - min((uint32_t)(c * 16.f), top);
+        key = (place << kb.cost) | q >> (kCostBits - kb.cost);
     }
     keys[p] = key | (reach > kLongWalk ? 0u : 1u << (kb.total - 1));
     idx[p] = (int32_t)p;

@@ -274,3 +274,20 @@ def test_batch_size_changes_no_result(ht, mode):
     assert torch.equal(one.pop("mask"), many.pop("mask"))
     for c, v in one.items():
         assert torch.equal(many[c].view(torch.int32), v.view(torch.int32).repeat(rep)), c
+
+
+def test_block_bits_change_no_result(ht):
+    """Every spatial block size that the tunable takes, from single cells to the whole tile."""
+    W = make_box_workload(ht, 64, 125.0, 20, 6, 2.0, 20.0, 7)
+    f, t, npk = W["finder"], W["tile"], W["npk"]
+    f.bind_fields(t["delta"], t["etax"], t["etay"], t["etaz"], t["eta2x"], t["eta2y"],
+                  t["eta2z"], None)
+    cost = torch.rand(npk, device="cuda", generator=torch.Generator("cuda").manual_seed(1)) * 300
+    want = None
+    for bits in (17, 0, 1, 5, 11, 12, 21, 40):
+        f.tune(block_bits=bits)
+        res = f.analyse(*W["args"], nbuff=20, mode="learned", cost=cost)
+        torch.cuda.synchronize()
+        res = {c: v.view(torch.int32).clone() for c, v in res.items()}
+        want = want or res
+        assert all(torch.equal(res[c], want[c]) for c in want), bits
