@@ -1099,7 +1099,8 @@ def run_collapse_table(args, rank, world, device):
             "roofline": None,
             "roofline_note": "latency-bound FP64 chains (one ellipsoid per thread, ~10^3 "
                              "dependent RK4 steps); no HBM or tensor-core bound applies",
-            "gpu_launches": args.steps, "clocks": ck,
+            # the evolution and the reciprocals of the growth table's spacings
+            "gpu_launches": 2 * args.steps, "clocks": ck,
             "e2e": {"value": world * n / e2e_s, "unit": "ellipsoids/s",
                     "h2d_bytes_per_step": 3 * n * 8 + 3 * ntab * 8,
                     "d2h_bytes_per_step": n * 8, "ms_per_step": 1e3 * e2e_s}}

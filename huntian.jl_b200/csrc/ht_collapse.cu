@@ -18,9 +18,10 @@
 // What is left of the RK4's time is the chain of its longest entries (10,000 dependent steps):
 // 0.45 warps per scheduler are resident on average, the FP64 pipe is 14 % busy and a warp waits
 // 1.4 cycles per instruction for the one before; taking the next round's roots before the
-// stopping test changed nothing.  This file is compiled with -fmad=false: no product is fused into an addition, the operations run in the
-// reference's order, and the one logarithm on the path (the oblate shape branch) is a
-// series both sides carry, so the results follow the CPU restatement to the last bit.
+// stopping test changed nothing.  This file is compiled with -fmad=false: no product is fused
+// into an addition, the operations run in the reference's order, and the one logarithm on the
+// path (the oblate shape branch) is a series both sides carry, so the results follow the CPU
+// restatement to the last bit.
 #include <cmath>
 #include <vector>
 

@@ -443,10 +443,13 @@ __global__ void __launch_bounds__(kEmitThreads) pf_emit_kernel(const uint32_t* _
 }
 
 // Count, scan and emit of a small grid in one launch: a CTA takes 256 words, one per thread,
-// and adds up the words before them itself (at most 256 KB from L2).  Three launches are
-// bound by their own latency there (2.7 + 3.3 + 5.2 us on a 128^3 region, 8 words in a row
-// per emitting thread; this one 9.4 us, and on a 48^3 region 3.8 against 13.8).  Counting
-// takes over above that size: the words before a CTA's grow with the square of the words.
+// and adds up the words before them itself (at most 256 KB from L2).  Three launches are bound
+// by their own latency and by eight words in a row per emitting thread.  The words before a
+// CTA's grow with the square of the words; peaks favour this form.  Whole scans, us, three
+// launches and this one: 48^3 cells 12.2 and 8.5, with 1,000 new peaks 20.6 and 12.4; 128^3
+// (65,536 words) 12.5 and 14.1 without new peaks, 14.8 and 14.7 with 185, 18.5 and 15.9 with
+// 6,400.  Over a bank of 30 filters the line lies between 65,536 words (464 and 454) and 92,480
+// (136^3 cells: 505 and 573).
 constexpr long long kSmallWords = 1 << 16;
 __global__ void __launch_bounds__(kEmitThreads) pf_emit_small_kernel(
     const uint32_t* __restrict__ bits, const PfEmit a, int64_t* count, int64_t* found) {

@@ -6,8 +6,8 @@
 // outward (the per-shell gather of ShellAnalysisGPU.jl:153-229 / ext/CUDAExt.jl:752-924):
 // each lane accumulates 13 sums per shell in FP64 from the FP32 cell values (delta,
 // delta*d, delta^T*d, and the symmetrised strain psi_L d_K + psi_K d_L, every product
-// exact in FP64); the lanes' partial sums are combined in FP64 in a fixed order by
-// exchanges, and the shell's profile (Fbar, gradients, strain) goes to a per-group
+// exact in FP64); the lanes' partial sums are combined in FP64 in a fixed order (by exchanges
+// or through shared memory, see combine), and the shell's profile (Fbar, gradients, strain) goes to a per-group
 // scratch slot in FP64.  The walk stops as
 // soon as every shell the post-processing reads has been gathered.  The same group then
 // runs the post-processing of RadialShell.jl:449-859 / ext/CUDAExt.jl:1213-1912 in FP64:

@@ -229,14 +229,17 @@ typedef struct {
     int64_t npeaks;
     /* Nullable: the order in which to process the peaks, a permutation of 0..npeaks-1
      * (entries outside that range are skipped).  Results stay indexed by peak, so any
-     * order gives identical results.  NULL: batch order (PLAIN), or a spatial order
-     * computed by the library (BATCHED: Morton order of (i, j, k) within each lane-group
-     * class, so that concurrently walked peaks share cells in L2). */
+     * order gives identical results.  NULL: batch order (PLAIN), or an order computed by the
+     * library (BATCHED): peaks whose walk reaches beyond 16 cells whatever the data, then
+     * the others, each in Morton order of (i, j, k), so that concurrently walked peaks share
+     * cells in L2. */
     const int32_t* order;
     /* Nullable: predicted cost per peak (the learned bracket's high quantile of the walk's
      * stop radius, ht_bracket_predict).  HT_MODE_LEARNED without a caller order processes
-     * the peaks by descending cost within each lane-group class, so that the peaks sharing
-     * a warp walk similar distances and the longest walks start first.  Ignored otherwise. */
+     * spatial blocks (HT_TUNE_BLOCK_BITS) one after the other and the peaks of a block by
+     * descending cost (in 1/16 cells, up to 256 cells), so that the peaks sharing a warp
+     * walk similar distances; peaks whose cost is above 16 cells go first, in the same order
+     * among themselves.  Ignored otherwise. */
     const float* cost;
 } ht_peak_batch;
 
@@ -304,9 +307,11 @@ HT_API int ht_shell_analyse_static(ht_ctx* ctx, const ht_fields* fields,
  * processing order.
  *   HT_TUNE_BLOCK_BITS  HT_MODE_LEARNED order: peaks are grouped into spatial blocks of
  *                       2^value cells (Morton prefix) and ordered by descending predicted
- *                       cost inside a block (default 17);
+ *                       cost inside a block (0 .. 40, default 17; smaller blocks leave the
+ *                       order's 32-bit keys fewer bits of the cost on sides above 512);
  *   HT_TUNE_PF_KZ       peak scan: k-planes per CTA (0 = chosen from the grid size);
- *   HT_TUNE_WALK_BPSM   shell walk: resident blocks per SM (0 = the occupancy maximum);
+ *   HT_TUNE_WALK_BPSM   shell walk: resident blocks per SM at most (0 = as many as fit: three,
+ *                       in BATCHED and LEARNED mode two below 180,000 peaks);
  *   HT_TUNE_FFT_PATH    ht_smooth_tile's inverse FFT: 0 = by tile side (the pencil passes
  *                       at 576 and 1152, one 3-D cuFFT plan for powers of two, otherwise
  *                       transposes + batched 1-D transforms), 1 = 3-D plan, 2 = transposed
